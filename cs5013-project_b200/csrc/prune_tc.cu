@@ -19,7 +19,12 @@
 //   4. thread t reads TMEM lane t (row t of G) and writes the bit mask of the
 //      candidates u that t, once chosen, prunes: alpha * d(t, u) <= d(node, u);
 //   5. one warp runs the sequential selection on bits only: p* = first live
-//      candidate, then the live set loses p*'s mask.  No row is fetched there.
+//      candidate, then the live set loses p*'s mask.  No row is fetched there.  A word
+//      of 32 candidates is decided from registers (lane i holds candidate i's bits
+//      within the word, one shuffle per p*), then each later word loses the OR of the
+//      chosen ones' masks; the list and its filter slots are written by all threads at
+//      the end.  Written inside the loop by one lane, the slots' 64-bit remainders were
+//      1,000 cycles per p*: 65k of a node's 77k cycles (1M-style build, 88 candidates).
 // Nodes with more than 256 candidates go to a second pass of the same kernel with
 // room for 512, larger ones to prune_kernel.  If the uint8 copy is not exact (a device flag written by
 // the conversion kernels) this kernel returns at once and prune_kernel does all.
@@ -112,7 +117,7 @@ __device__ __forceinline__ uint32_t dp4a_u(uint32_t a, uint32_t b, uint32_t c) {
 
 // shared memory of one CTA handling up to maxc candidates per node
 struct TcLayout {
-    uint32_t rows, nodev, cid, cd, keys, perm, sid, sd, nrm, pm, bmask, bar, misc, bytes;
+    uint32_t rows, nodev, cid, cd, keys, perm, sid, sd, nrm, pm, bmask, chosen, bar, misc, bytes;
     __host__ __device__ static TcLayout make(uint32_t D, uint32_t maxc) {
         TcLayout l;
         l.rows  = 0;                  // maxc x D bytes, canonical layout, sorted order
@@ -126,8 +131,9 @@ struct TcLayout {
         l.nrm   = l.sd + 4 * maxc;
         l.pm    = l.nrm + 4 * maxc;   // [maxc][maxc / 32] prune masks
         l.bmask = l.pm + maxc * maxc / 8;  // sorted positions holding B candidates
-        l.bar   = l.bmask + maxc / 8;
-        l.misc  = l.bar + 8;
+        l.chosen = l.bmask + maxc / 8;  // the node's new list
+        l.bar    = l.chosen + 4 * kMaxR;
+        l.misc   = l.bar + 8;
         l.bytes = l.misc + 4 * 16;
         return l;
     }
@@ -167,7 +173,8 @@ __global__ void __launch_bounds__(kThreads) prune_tc_kernel(PruneArgs a, uint32_
     uint32_t*      nrm   = reinterpret_cast<uint32_t*>(smem + lay.nrm);
     uint32_t*      pm    = reinterpret_cast<uint32_t*>(smem + lay.pm);
     uint32_t*      bmask = reinterpret_cast<uint32_t*>(smem + lay.bmask);
-    uint32_t*      misc  = reinterpret_cast<uint32_t*>(smem + lay.misc);  // [0] tmem, [2..13] work items
+    uint32_t*      chosen = reinterpret_cast<uint32_t*>(smem + lay.chosen);
+    uint32_t*      misc  = reinterpret_cast<uint32_t*>(smem + lay.misc);  // [0] tmem, [1] degree, [2..13] work items
     const uint32_t bar    = saddr(smem + lay.bar);
     const uint32_t rows_s = saddr(rows);
 
@@ -418,6 +425,11 @@ __global__ void __launch_bounds__(kThreads) prune_tc_kernel(PruneArgs a, uint32_
             }
             if (failed) break;
             if (t < m) {
+                // consistent lists: no B candidate is checked against another
+                if (a.consistent && ((bmask[t >> 5] >> (t & 31u)) & 1u)) {
+#pragma unroll
+                    for (uint32_t q = 0; q < QW; ++q) mk[q] &= ~bmask[q];
+                }
                 uint4* dst = reinterpret_cast<uint4*>(pm + t * QW);
 #pragma unroll
                 for (uint32_t q = 0; q < QW / 4; ++q)
@@ -428,88 +440,46 @@ __global__ void __launch_bounds__(kThreads) prune_tc_kernel(PruneArgs a, uint32_
         tc_fence_before();
         __syncthreads();
 
-        // --- 7. sequential selection on bits (warp 0): lane q holds live-set word q
+        // --- 7. sequential selection on bits (warp 0), a word of 32 candidates at a time
         if (warp == 0) {
-            uint32_t live = 0u;
+            uint32_t live = 0u;  // lane q holds live-set word q
             if (lane < QW && m > 32u * lane) {
                 const uint32_t left = m - 32u * lane;
                 live                = left >= 32u ? ~0u : (1u << left) - 1u;
             }
-            uint64_t       out  = (uint64_t)node * R;
-            uint32_t       ndeg = 0;
-            auto emit = [&](uint32_t t, uint32_t slot) {
-                const uint32_t id = sid[t];
-                a.adj[out + slot]   = id;
-                a.adj_h[out + slot] = bloom_pack(id);
-            };
-            if (!a.consistent) {
-                // one round per chosen neighbour
-                while (ndeg < R) {
-                    const uint32_t bm = __ballot_sync(0xffffffffu, live != 0u);
-                    if (bm == 0u) break;
-                    const uint32_t k0 = __ffs(bm) - 1u;
-                    const uint32_t wv = __shfl_sync(0xffffffffu, live, k0);
-                    const uint32_t t  = 32u * k0 + __ffs(wv) - 1u;
-                    if (lane == 0) emit(t, ndeg);
-                    ++ndeg;
-                    if (ndeg >= R) break;
-                    if (lane < QW) live &= ~pm[t * QW + lane];
-                    if (lane == k0) live &= ~(1u << (t & 31u));
+            uint32_t       ndeg  = 0;
+            const uint32_t words = (m + 31u) / 32u;
+            for (uint32_t k = 0; k < words && ndeg < R; ++k) {
+                uint32_t       wv  = __shfl_sync(0xffffffffu, live, k);
+                const uint32_t row = pm[(32u * k + lane) * QW + k];  // row t's bits within the word
+                uint32_t       got = 0u;
+                // p* = first live candidate; it and what it prunes leave the word
+                for (uint32_t room = R - ndeg; wv != 0u && room != 0u; --room) {
+                    const uint32_t t = __ffs(wv) - 1u;
+                    got |= 1u << t;
+                    wv &= ~(__shfl_sync(0xffffffffu, row, t) | (1u << t));
                 }
-            } else {
-                // B came out of RobustPrune with this alpha, so no B candidate prunes
-                // another: every live B candidate before the next live A candidate is
-                // chosen in one step, then that A candidate is decided.
-                const uint32_t bw = lane < QW ? bmask[lane] : 0u;
-                while (ndeg < R) {
-                    const uint32_t aw  = live & ~bw;
-                    const uint32_t bmA = __ballot_sync(0xffffffffu, aw != 0u);
-                    uint32_t       tA  = m;
-                    if (bmA) {
-                        const uint32_t k = __ffs(bmA) - 1u;
-                        tA               = 32u * k + __ffs(__shfl_sync(0xffffffffu, aw, k)) - 1u;
-                    }
-                    uint32_t run = 0u;
-                    if (lane < QW) {
-                        const uint32_t lo     = 32u * lane;
-                        const uint32_t before = tA >= lo + 32u ? ~0u : (tA <= lo ? 0u : (1u << (tA - lo)) - 1u);
-                        run                   = live & bw & before;
-                    }
-                    const uint32_t cnt = __popc(run);
-                    uint32_t       inc = cnt;  // inclusive prefix over lanes
-#pragma unroll
-                    for (uint32_t o = 1; o < 32; o <<= 1) {
-                        const uint32_t v = __shfl_up_sync(0xffffffffu, inc, o);
-                        if (lane >= o) inc += v;
-                    }
-                    const uint32_t total = __shfl_sync(0xffffffffu, inc, 31);
-                    const uint32_t take  = min(total, R - ndeg);
-                    uint32_t       j     = inc - cnt;
-                    for (uint32_t bits = run; bits != 0u && j < take; bits &= bits - 1u, ++j)
-                        emit(32u * lane + __ffs(bits) - 1u, ndeg + j);
-                    ndeg += take;
-                    if (ndeg >= R) break;
-                    live &= ~run;
-                    uint32_t acc = 0u;  // everything the run prunes
-                    for (uint32_t q = 0; q < QW; ++q) {
-                        for (uint32_t rq = __shfl_sync(0xffffffffu, run, q); rq != 0u; rq &= rq - 1u) {
-                            const uint32_t t = 32u * q + __ffs(rq) - 1u;
-                            if (lane < QW) acc |= pm[t * QW + lane];
-                        }
-                    }
-                    live &= ~acc;
-                    if (tA >= m) break;  // every live candidate was in the run
-                    const uint32_t tw = __shfl_sync(0xffffffffu, live, tA >> 5);
-                    if ((tw >> (tA & 31u)) & 1u) {
-                        if (lane == 0) emit(tA, ndeg);
-                        ++ndeg;
-                        if (ndeg >= R) break;
-                        if (lane < QW) live &= ~pm[tA * QW + lane];
-                        if (lane == (tA >> 5)) live &= ~(1u << (tA & 31u));
-                    }
+                const bool mine = (got >> lane) & 1u;
+                if (mine) chosen[ndeg + __popc(got & ((1u << lane) - 1u))] = sid[32u * k + lane];
+                ndeg += __popc(got);
+                // the later words lose what the word's chosen candidates prune
+                for (uint32_t q = k + 1u; q < words; ++q) {
+                    const uint32_t out =
+                        __reduce_or_sync(0xffffffffu, mine ? pm[(32u * k + lane) * QW + q] : 0u);
+                    if (lane == q) live &= ~out;
                 }
             }
-            if (lane == 0) a.deg[node] = ndeg;
+            if (lane == 0) {
+                misc[1]     = ndeg;
+                a.deg[node] = ndeg;
+            }
+        }
+        __syncthreads();
+        // the new list and its filter slots, one entry per thread
+        if (tid < misc[1]) {
+            const uint32_t id                 = chosen[tid];
+            a.adj[(uint64_t)node * R + tid]   = id;
+            a.adj_h[(uint64_t)node * R + tid] = bloom_pack(id);
         }
         ++done;
     }
