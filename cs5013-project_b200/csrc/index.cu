@@ -407,8 +407,6 @@ struct vann_index {
         }
     }
 
-    // RobustPrune launch: the tensor-core pass when an exact uint8 copy exists
-    // (decided on the device by the exactness flag), prune_kernel for the rest
     // RobustPrune launch.  Consistent reverse re-prunes go first to the warp-per-node
     // kernel; the tensor-core passes take what it hands on (or every node) when an
     // exact uint8 copy may exist (decided on the device by the exactness flag);
@@ -441,7 +439,7 @@ struct vann_index {
         }
         if (tc) {
             uint32_t* tc_counters = next_counter(st);  // one per pass
-            VCHECK(cudaMemsetAsync(tc_counters + 1, 0, 2 * sizeof(uint32_t), st));
+            VCHECK(cudaMemsetAsync(tc_counters + 1, 0, 3 * sizeof(uint32_t), st));
             VCHECK(vann::launch_prune_tc(pa, in_list, in_count, last_list, last_count, ws, tc_counters, num_sms,
                                          st));
             in_list  = last_list;

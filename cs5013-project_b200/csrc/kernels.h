@@ -95,7 +95,7 @@ struct PruneArgs {
 cudaError_t launch_prune(const PruneArgs& a, int num_sms, cudaStream_t st);
 bool        prune_tc_supported(uint32_t D, uint32_t R);
 // Tensor-core passes over in_list (every node when null); leftovers to out_list.
-// ws: 2 * n_nodes + 4 words of scratch; counters: three zeroed work counters.
+// ws: 2 * n_nodes + 4 words of scratch; counters: four zeroed work counters.
 cudaError_t launch_prune_tc(const PruneArgs& a, const uint32_t* in_list, const uint32_t* in_count,
                             uint32_t* out_list, uint32_t* out_count, uint32_t* ws, uint32_t* counters, int num_sms,
                             cudaStream_t st);

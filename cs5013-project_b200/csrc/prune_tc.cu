@@ -7,27 +7,30 @@
 // sums in any order, and the integer identity |x|^2 + |y|^2 - 2 x.y, give the
 // same value: the decisions are bit-identical to the FP32 path.
 //
-// One CTA of 4 warps prunes one node at a time:
+// One CTA of 4 warps (the 128 TMEM lanes) prunes one node at a time:
 //   1. candidate ids (A then B, as in prune.cu) with their distances to the node
 //      (given by the search, or computed exactly from the uint8 rows);
-//   2. stable order by (distance, candidate index): each key's rank is the count
-//      of smaller keys (one pass, one barrier);
+//   2. stable order by (distance, candidate index): a candidate's rank is the count of
+//      the distances below its own, equal ones of lower index included;
 //   3. the first `cap` candidates' uint8 rows are staged in shared memory in that
 //      order, in the K-major no-swizzle layout tcgen05.mma reads (8-row x 16-byte
 //      core matrices), and one thread issues tcgen05.mma.kind::i8 (u8 x u8 -> s32)
-//      for the Gram matrix G = C C^T into tensor memory (TMEM), 128 x <= 128 per tile;
-//   4. thread t reads TMEM lane t (row t of G) and writes the bit mask of the
-//      candidates u that t, once chosen, prunes: alpha * d(t, u) <= d(node, u);
-//   5. one warp runs the sequential selection on bits only: p* = first live
-//      candidate, then the live set loses p*'s mask.  No row is fetched there.  A word
-//      of 32 candidates is decided from registers (lane i holds candidate i's bits
-//      within the word, one shuffle per p*), then each later word loses the OR of the
-//      chosen ones' masks; the list and its filter slots are written by all threads at
-//      the end.  Written inside the loop by one lane, the slots' 64-bit remainders were
-//      1,000 cycles per p*: 65k of a node's 77k cycles (1M-style build, 88 candidates).
-// Nodes with more than 256 candidates go to a second pass of the same kernel with
-// room for 512, larger ones to prune_kernel.  If the uint8 copy is not exact (a device flag written by
-// the conversion kernels) this kernel returns at once and prune_kernel does all.
+//      for the Gram matrix G = C C^T into tensor memory (TMEM), tile by tile;
+//   4. thread t reads TMEM lane t (row t of G, which is its column t) and writes the
+//      bits of the earlier candidates u that, once chosen, prune t: alpha * d(u, t) <=
+//      d(node, t).  Only the tiles on and below the diagonal are computed;
+//   5. one warp decides the candidates on those bits, 32 at a time: a candidate is out
+//      when a chosen one of an earlier word prunes it; within the word every candidate
+//      with no undecided pruner is chosen, what those prune is out, and so on (a few
+//      rounds of two ballots, where one p* after the other took a shuffle each);
+//   6. all threads write the list and its filter slots.
+// The phases are short dependent chains (loads, barriers, ballots), so what bounds the
+// kernel is how many nodes an SM has in flight: up to 128 candidates a CTA takes 64
+// TMEM columns and fits 8 times (tiles of 128 x 64), larger classes 128 columns, 4 at
+// most.  Nodes with more candidates than a pass holds go to the next pass (256, 512,
+// 768), larger ones to prune_kernel.  If the uint8 copy is not exact (a device flag
+// written by the conversion kernels) this kernel returns at once and prune_kernel does
+// all.
 #include "common.cuh"
 #include "kernels.h"
 
@@ -35,7 +38,6 @@ namespace vann {
 namespace {
 
 constexpr uint32_t kThreads  = 128;  // 4 warps = the 128 TMEM lanes
-constexpr uint32_t kTmemCols = 128;  // accumulator columns per CTA
 constexpr uint32_t kMaxR     = 128;
 constexpr long long kSpinCycles = 2000000000ll;  // ~1 s bound on an MMA completion wait
 
@@ -117,39 +119,35 @@ __device__ __forceinline__ uint32_t dp4a_u(uint32_t a, uint32_t b, uint32_t c) {
 
 // shared memory of one CTA handling up to maxc candidates per node
 struct TcLayout {
-    uint32_t rows, nodev, cid, cd, keys, perm, sid, sd, nrm, pm, bmask, chosen, bar, misc, bytes;
+    uint32_t rows, nodev, cid, cd, sid, sd, nrm, pby, bmask, chosen, bar, misc, bytes;
     __host__ __device__ static TcLayout make(uint32_t D, uint32_t maxc) {
         TcLayout l;
-        l.rows  = 0;                  // maxc x D bytes, canonical layout, sorted order
-        l.nodev = l.rows + maxc * D;  // D bytes
-        l.cid   = l.nodev + ((D + 15) & ~15u);
-        l.cd    = l.cid + 4 * maxc;   // candidate order (A then B)
-        l.keys  = l.cd + 4 * maxc;    // 8-byte aligned: every offset above is a multiple of 16
-        l.perm  = l.keys + 8 * maxc;  // sorted position -> candidate index
-        l.sid   = l.perm + 4 * maxc;  // ids, distances, squared norms in sorted order
-        l.sd    = l.sid + 4 * maxc;
-        l.nrm   = l.sd + 4 * maxc;
-        l.pm    = l.nrm + 4 * maxc;   // [maxc][maxc / 32] prune masks
-        l.bmask = l.pm + maxc * maxc / 8;  // sorted positions holding B candidates
-        l.chosen = l.bmask + maxc / 8;  // the node's new list
+        l.rows   = 0;                  // maxc x D bytes, canonical layout, sorted order
+        l.nodev  = l.rows + maxc * D;  // D bytes
+        l.cid    = l.nodev + ((D + 15) & ~15u);
+        l.cd     = l.cid + 4 * maxc;  // candidate order (A then B)
+        l.sid    = l.cd + 4 * maxc;   // sorted order: id (top bit: a B candidate), distance,
+        l.sd     = l.sid + 4 * maxc;  // squared norm
+        l.nrm    = l.sd + 4 * maxc;
+        l.pby    = l.nrm + 4 * maxc;  // [maxc / 32][maxc] bits of the candidates that prune t
+        l.bmask  = l.pby + maxc * maxc / 8;  // sorted positions holding B candidates
+        l.chosen = l.bmask + maxc / 8;       // the node's new list
         l.bar    = l.chosen + 4 * kMaxR;
         l.misc   = l.bar + 8;
-        l.bytes = l.misc + 4 * 16;
+        l.bytes  = l.misc + 4 * 16;
         return l;
     }
 };
 
-__device__ __forceinline__ uint64_t u64_of(uint32_t lo, uint32_t hi) { return ((uint64_t)hi << 32) | lo; }
-
 // Nodes are the slots in_list[0 .. *in_count) (or 0 .. n_nodes when in_list is
-// null); nodes with more than MAXC candidates go to out_list.
-template <uint32_t MAXC>
-__global__ void __launch_bounds__(kThreads) prune_tc_kernel(PruneArgs a, uint32_t* counter, const uint32_t* in_list,
-                                                            const uint32_t* in_count, uint32_t* out_list,
-                                                            uint32_t* out_count) {
-    constexpr uint32_t QW  = MAXC / 32;        // mask words per candidate
-    constexpr uint32_t NB  = MAXC / 128;       // 128-row blocks
-    constexpr uint32_t KPT = MAXC / kThreads;  // sort keys per thread
+// null); nodes with more than MAXC candidates go to out_list.  COLS: TMEM columns per
+// CTA, the width of a Gram tile.
+template <uint32_t MAXC, uint32_t COLS>
+__global__ void __launch_bounds__(kThreads, MAXC == 128 ? 8 : 1)
+    prune_tc_kernel(PruneArgs a, uint32_t* counter, const uint32_t* in_list, const uint32_t* in_count,
+                    uint32_t* out_list, uint32_t* out_count) {
+    constexpr uint32_t KPT = MAXC / kThreads;  // candidates per thread
+    constexpr uint32_t kB  = 0x80000000u;      // sid: a B candidate (ids are below 2^31)
     extern __shared__ __align__(1024) unsigned char smem[];
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     const uint64_t nwork = in_list ? (uint64_t)*reinterpret_cast<volatile const uint32_t*>(in_count) : a.n_nodes;
@@ -162,25 +160,23 @@ __global__ void __launch_bounds__(kThreads) prune_tc_kernel(PruneArgs a, uint32_
 
     const uint32_t D = a.D, R = a.R;
     const TcLayout lay = TcLayout::make(D, MAXC);
-    unsigned char* rows  = smem + lay.rows;
-    uint8_t*       nodev = smem + lay.nodev;
-    uint32_t*      cid   = reinterpret_cast<uint32_t*>(smem + lay.cid);
-    float*         cd    = reinterpret_cast<float*>(smem + lay.cd);
-    uint64_t*      keys  = reinterpret_cast<uint64_t*>(smem + lay.keys);
-    uint32_t*      perm  = reinterpret_cast<uint32_t*>(smem + lay.perm);
-    uint32_t*      sid   = reinterpret_cast<uint32_t*>(smem + lay.sid);
-    float*         sd    = reinterpret_cast<float*>(smem + lay.sd);
-    uint32_t*      nrm   = reinterpret_cast<uint32_t*>(smem + lay.nrm);
-    uint32_t*      pm    = reinterpret_cast<uint32_t*>(smem + lay.pm);
-    uint32_t*      bmask = reinterpret_cast<uint32_t*>(smem + lay.bmask);
+    unsigned char* rows   = smem + lay.rows;
+    uint8_t*       nodev  = smem + lay.nodev;
+    uint32_t*      cid    = reinterpret_cast<uint32_t*>(smem + lay.cid);
+    float*         cd     = reinterpret_cast<float*>(smem + lay.cd);
+    uint32_t*      sid    = reinterpret_cast<uint32_t*>(smem + lay.sid);
+    float*         sd     = reinterpret_cast<float*>(smem + lay.sd);
+    uint32_t*      nrm    = reinterpret_cast<uint32_t*>(smem + lay.nrm);
+    uint32_t*      pby    = reinterpret_cast<uint32_t*>(smem + lay.pby);
+    uint32_t*      bmask  = reinterpret_cast<uint32_t*>(smem + lay.bmask);
     uint32_t*      chosen = reinterpret_cast<uint32_t*>(smem + lay.chosen);
-    uint32_t*      misc  = reinterpret_cast<uint32_t*>(smem + lay.misc);  // [0] tmem, [1] degree, [2..13] work items
+    uint32_t*      misc   = reinterpret_cast<uint32_t*>(smem + lay.misc);  // [0] tmem, [1] degree, [2..13] work items
     const uint32_t bar    = saddr(smem + lay.bar);
     const uint32_t rows_s = saddr(rows);
 
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(saddr(misc)),
-                     "r"(kTmemCols));
+                     "r"(COLS));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     if (tid == 0) {
@@ -194,6 +190,7 @@ __global__ void __launch_bounds__(kThreads) prune_tc_kernel(PruneArgs a, uint32_
 
     const bool     rev    = a.csr_off != nullptr;
     const uint32_t nchunk = D / 16;
+    const uint32_t inv_nc = 0xFFFFFFFFu / nchunk + 1u;  // x / nchunk = __umulhi(x, inv_nc), nchunk >= 2
     const uint32_t LBO = 128, SBO = 8 * D;  // 8 rows x 16 B per core matrix; chunks adjacent
     const uint32_t ksteps = D / 32;         // kind::i8: K = 32 per instruction
     uint32_t       phase  = 0;
@@ -263,13 +260,14 @@ __global__ void __launch_bounds__(kThreads) prune_tc_kernel(PruneArgs a, uint32_
             cid[i] = id;
             cd[i]  = d;
         }
-        if (computed && tid < nchunk)
-            *reinterpret_cast<uint4*>(nodev + 16 * tid) =
-                __ldg(reinterpret_cast<const uint4*>(a.vecs_u8 + (uint64_t)node * D) + tid);
-        __syncthreads();
-
-        // --- 2. missing distances straight from the uint8 rows (exact integers)
+        if (tid < 3u && nc + tid < MAXC)  // groups of four below read past an uneven count
+            cd[nc + tid] = __uint_as_float(0xFFFFFFFFu);
         if (computed) {
+            if (tid < nchunk)
+                *reinterpret_cast<uint4*>(nodev + 16 * tid) =
+                    __ldg(reinterpret_cast<const uint4*>(a.vecs_u8 + (uint64_t)node * D) + tid);
+            __syncthreads();
+            // missing distances straight from the uint8 rows (exact integers)
             uint32_t nn = 0;  // |node|^2
             for (uint32_t c = 0; c < nchunk; ++c) {
                 const uint4 q = *reinterpret_cast<const uint4*>(nodev + 16 * c);
@@ -288,69 +286,83 @@ __global__ void __launch_bounds__(kThreads) prune_tc_kernel(PruneArgs a, uint32_
                 cd[i] = (float)(nn + n - 2u * dot);
             }
         }
-        for (uint32_t i = tid; i < nc; i += kThreads) keys[i] = make_key(cd[i], i);
-        if (tid == 0 && (nc & 1u)) keys[nc] = ~0ull;  // pairs below read one past an odd count
         __syncthreads();
 
-        // --- 3. stable order by (distance, candidate index): rank = keys below
+        // --- 2. stable order by (distance, candidate index).  Distances are non-negative,
+        // so their bits order them; index i = 128 q + tid counts equal bits of lower index.
+        const uint32_t m = min(nc, a.cap);
         {
-            uint64_t k[KPT];
-            uint32_t r[KPT];
+            uint32_t b[KPT], r[KPT];
 #pragma unroll
             for (uint32_t q = 0; q < KPT; ++q) {
                 const uint32_t i = tid + q * kThreads;
-                k[q]             = i < nc ? keys[i] : ~0ull;
+                b[q]             = i < nc ? __float_as_uint(cd[i]) : 0u;
                 r[q]             = 0;
             }
-            const uint32_t used = (nc + kThreads - 1) / kThreads;  // key slots in use per thread
-            for (uint32_t j = 0; j < nc; j += 2) {
-                const uint4    kk = *reinterpret_cast<const uint4*>(keys + j);
-                const uint64_t x = u64_of(kk.x, kk.y), y = u64_of(kk.z, kk.w);
+            const uint32_t used = (nc + kThreads - 1) / kThreads;  // candidates in use per thread
+            for (uint32_t c0 = 0; c0 < nc; c0 += 32) {             // the warp's own chunk: 128 q + 32 warp
 #pragma unroll
-                for (uint32_t q = 0; q < KPT; ++q)
-                    if (q < used) r[q] += (uint32_t)(x < k[q]) + (uint32_t)(y < k[q]);
+                for (uint32_t q = 0; q < KPT; ++q) {
+                    if (q >= used) break;
+                    const uint32_t own = 128u * q + 32u * warp;
+                    const uint4*   dj  = reinterpret_cast<const uint4*>(cd + c0);
+                    const uint32_t n4  = min(8u, (nc - c0 + 3u) / 4u);
+                    if (c0 != own) {
+                        const uint32_t thr = b[q] + (c0 < own ? 1u : 0u);
+                        for (uint32_t j = 0; j < n4; ++j) {
+                            const uint4 x = dj[j];
+                            r[q] += (uint32_t)(x.x < thr) + (uint32_t)(x.y < thr) + (uint32_t)(x.z < thr) +
+                                    (uint32_t)(x.w < thr);
+                        }
+                    } else {
+                        for (uint32_t j = 0; j < n4; ++j) {
+                            const uint4 x = dj[j];
+                            r[q] += (uint32_t)(x.x < b[q] + (4u * j < lane ? 1u : 0u)) +
+                                    (uint32_t)(x.y < b[q] + (4u * j + 1u < lane ? 1u : 0u)) +
+                                    (uint32_t)(x.z < b[q] + (4u * j + 2u < lane ? 1u : 0u)) +
+                                    (uint32_t)(x.w < b[q] + (4u * j + 3u < lane ? 1u : 0u));
+                        }
+                    }
+                }
             }
 #pragma unroll
             for (uint32_t q = 0; q < KPT; ++q) {
                 const uint32_t i = tid + q * kThreads;
-                if (i < nc) perm[r[q]] = i;
+                if (i < nc && r[q] < m) {
+                    sid[r[q]] = cid[i] | (i >= nA ? kB : 0u);
+                    sd[r[q]]  = __uint_as_float(b[q]);
+                }
             }
         }
         __syncthreads();
 
-        // --- 4. the first ncap candidates in sorted order: rows staged for the MMA
-        const uint32_t m = min(nc, a.cap);
-#pragma unroll
-        for (uint32_t q = 0; q < NB; ++q) {
-            const uint32_t t = 128u * q + tid;
-            bool           b = false;
-            if (t < m) {
-                const uint32_t i = perm[t];
-                sid[t]           = cid[i];
-                sd[t]            = cd[i];
-                b                = i >= nA;
-            }
-            const uint32_t bits = __ballot_sync(0xffffffffu, b);
-            if (lane == 0) bmask[4u * q + warp] = bits;
-        }
+        // --- 3. the first `cap` candidates' rows staged for the MMA
         for (uint32_t x = tid; x < m * nchunk; x += kThreads) {
-            const uint32_t t = x / nchunk, c = x - t * nchunk;
+            const uint32_t t = __umulhi(x, inv_nc), c = x - t * nchunk;
             cp_async16(rows_s + (t >> 3) * SBO + c * LBO + (t & 7u) * 16u,
-                       a.vecs_u8 + (uint64_t)cid[perm[t]] * D + 16u * c);
+                       a.vecs_u8 + (uint64_t)(sid[t] & ~kB) * D + 16u * c);
+        }
+        if (a.consistent) {
+#pragma unroll
+            for (uint32_t q = 0; q < KPT; ++q) {
+                const uint32_t t    = 128u * q + tid;
+                const uint32_t bits = __ballot_sync(0xffffffffu, t < m && (sid[t] & kB) != 0u);
+                if (lane == 0) bmask[4u * q + warp] = bits;
+            }
         }
         cp_async_wait_all();
         fence_proxy_async();  // rows become visible to the tensor core's reads
         __syncthreads();
 
-        // --- 5. Gram tiles on the tensor cores; squared norms of the staged rows
-        const uint32_t nb = (m + 127u) / 128u;  // row / column blocks of 128
+        // --- 4. Gram tiles on the tensor cores; squared norms of the staged rows
+        const uint32_t nb = (m + 127u) / 128u;  // row blocks of 128
         auto issue_tile = [&](uint32_t r, uint32_t c) {
-            const uint32_t left = m - 128u * c;
-            const uint32_t N    = ((left < 128u ? left : 128u) + 15u) & ~15u;
+            const uint32_t left = m - COLS * c;
+            const uint32_t N    = ((left < COLS ? left : COLS) + 15u) & ~15u;
             const uint32_t id   = idesc_u8(128u, N);
             for (uint32_t s = 0; s < ksteps; ++s) {
                 const uint64_t da = umma_desc(rows_s + r * 16u * SBO + s * 2u * LBO, LBO, SBO);
-                const uint64_t db = umma_desc(rows_s + c * 16u * SBO + s * 2u * LBO, LBO, SBO);
+                const uint64_t db = umma_desc(rows_s + c * (COLS / 8u) * SBO + s * 2u * LBO, LBO, SBO);
                 mma_u8(tmem, da, db, id, s > 0 ? 1u : 0u);
             }
             mma_commit(bar);
@@ -366,108 +378,99 @@ __global__ void __launch_bounds__(kThreads) prune_tc_kernel(PruneArgs a, uint32_
                 n = dp4a_u(v.x, v.x, dp4a_u(v.y, v.y, dp4a_u(v.z, v.z, dp4a_u(v.w, v.w, n))));
             }
             nrm[t] = n;
-            // "t prunes u" is alpha * d(t, u) <= d(node, u) in FP32, with d(t, u) the exact
-            // integer Y = |t|^2 + |u|^2 - 2 t.u (< 2^24, so FP32 holds it exactly).  fl(Y *
-            // alpha) does not decrease as Y grows, so the test is Y <= Ymax(u), the largest
-            // integer with fl(Ymax * alpha) <= d(node, u): 2 t.u - |t|^2 >= |u|^2 - Ymax(u).
-            // That threshold replaces d(node, u) in the same slot.
-            const float sdt = sd[t];
-            int         y   = (int)fminf(floorf(sdt / a.alpha), 16777215.f);
-            while (y < 16777215 && (float)(y + 1) * a.alpha <= sdt) ++y;
-            while (y > 0 && (float)y * a.alpha > sdt) --y;
-            reinterpret_cast<int*>(sd)[t] = (int)n - y;
         }
         __syncthreads();
-        const int* thr = reinterpret_cast<const int*>(sd);
 
-        // --- 6. prune masks in sorted order: bit u of row t = "t, once chosen, prunes u"
+        // --- 5. bits of the candidates that prune t
         for (uint32_t r = 0; r < nb; ++r) {
-            const uint32_t t  = 128u * r + tid;
-            const int      nt = t < m ? (int)nrm[t] : 0;
-            uint32_t       mk[QW];
-#pragma unroll
-            for (uint32_t q = 0; q < QW; ++q) mk[q] = 0u;
-#pragma unroll
-            for (uint32_t c = 0; c < NB; ++c) {
-                if (c < nb) {
-                    if (r != 0 || c != 0) {
-                        tc_fence_before();
-                        __syncthreads();  // every thread's reads of the previous tile are done
-                        if (tid == 0) {
-                            tc_fence_after();
-                            issue_tile(r, c);
-                        }
+            const uint32_t t = 128u * r + tid;
+            // "u prunes t" is alpha * d(u, t) <= d(node, t) in FP32, with d(u, t) the exact
+            // integer Y = |u|^2 + |t|^2 - 2 u.t (< 2^24, so FP32 holds it exactly).  fl(Y *
+            // alpha) does not decrease as Y grows, so the test is Y <= Ymax(t), the largest
+            // integer with fl(Ymax * alpha) <= d(node, t): 2 u.t - |u|^2 >= |t|^2 - Ymax(t).
+            int      thr  = 0;
+            uint32_t keep = ~0u;  // consistent lists: no B candidate is checked against another
+            if (t < m) {
+                const float sdt = sd[t];
+                int         y   = (int)fminf(floorf(sdt / a.alpha), 16777215.f);
+                while (y < 16777215 && (float)(y + 1) * a.alpha <= sdt) ++y;
+                while (y > 0 && (float)y * a.alpha > sdt) --y;
+                thr = (int)nrm[t] - y;
+                if (a.consistent && (sid[t] & kB)) keep = 0u;
+            }
+            const uint32_t last  = 128u * r + 32u * warp + 31u;  // the warp's last candidate
+            const uint32_t ncols = min(m, 128u * (r + 1u));
+            for (uint32_t c = 0; COLS * c < ncols; ++c) {
+                if (r != 0 || c != 0) {
+                    tc_fence_before();
+                    __syncthreads();  // every thread's reads of the previous tile are done
+                    if (tid == 0) {
+                        tc_fence_after();
+                        issue_tile(r, c);
                     }
-                    const bool ok = mbar_wait(bar, phase);
-                    phase ^= 1u;
-                    if (__syncthreads_or(!ok)) {
-                        failed = true;
-                        break;
-                    }
-                    tc_fence_after();
-                    const uint32_t left = m - 128u * c;
-                    const uint32_t N    = ((left < 128u ? left : 128u) + 15u) & ~15u;
+                }
+                const bool ok = mbar_wait(bar, phase);
+                phase ^= 1u;
+                if (__syncthreads_or(!ok)) {
+                    failed = true;
+                    break;
+                }
+                tc_fence_after();
+#pragma unroll 1
+                for (uint32_t c32 = 0; c32 < COLS; c32 += 32u) {
+                    const uint32_t u0 = COLS * c + c32;
+                    if (u0 >= m || u0 > last) break;
+                    uint32_t word = 0;
 #pragma unroll
-                    for (uint32_t c16 = 0; c16 < 128u; c16 += 16u) {
-                        if (c16 < N) {
+                    for (uint32_t h = 0; h < 32u; h += 16u) {
+                        if (u0 + h < m) {
                             uint32_t g[16];
-                            tmem_ld16(tmem + ((32u * warp) << 16) + c16, g);
-                            uint32_t bits = 0;
+                            tmem_ld16(tmem + ((32u * warp) << 16) + c32 + h, g);
 #pragma unroll
-                            for (uint32_t k = 0; k < 16; ++k) {
-                                const uint32_t u = 128u * c + c16 + k;
-                                bits |= (uint32_t)((int)(2u * g[k]) - nt >= thr[u]) << k;
+                            for (uint32_t k = 0; k < 16; k += 4) {
+                                const uint4 nu = *reinterpret_cast<const uint4*>(nrm + u0 + h + k);
+                                word |= (uint32_t)((int)(2u * g[k] - nu.x) >= thr) << (h + k);
+                                word |= (uint32_t)((int)(2u * g[k + 1] - nu.y) >= thr) << (h + k + 1);
+                                word |= (uint32_t)((int)(2u * g[k + 2] - nu.z) >= thr) << (h + k + 2);
+                                word |= (uint32_t)((int)(2u * g[k + 3] - nu.w) >= thr) << (h + k + 3);
                             }
-                            mk[4u * c + (c16 >> 5)] |= bits << (c16 & 16u);
                         }
                     }
+                    if (keep == 0u) word &= ~bmask[u0 >> 5];
+                    if (t < m) pby[(u0 >> 5) * MAXC + t] = word;
                 }
             }
             if (failed) break;
-            if (t < m) {
-                // consistent lists: no B candidate is checked against another
-                if (a.consistent && ((bmask[t >> 5] >> (t & 31u)) & 1u)) {
-#pragma unroll
-                    for (uint32_t q = 0; q < QW; ++q) mk[q] &= ~bmask[q];
-                }
-                uint4* dst = reinterpret_cast<uint4*>(pm + t * QW);
-#pragma unroll
-                for (uint32_t q = 0; q < QW / 4; ++q)
-                    dst[q] = make_uint4(mk[4 * q], mk[4 * q + 1], mk[4 * q + 2], mk[4 * q + 3]);
-            }
         }
         if (failed) break;
         tc_fence_before();
         __syncthreads();
 
-        // --- 7. sequential selection on bits (warp 0), a word of 32 candidates at a time
+        // --- 6. selection (warp 0), a word of 32 candidates at a time
         if (warp == 0) {
-            uint32_t live = 0u;  // lane q holds live-set word q
-            if (lane < QW && m > 32u * lane) {
-                const uint32_t left = m - 32u * lane;
-                live                = left >= 32u ? ~0u : (1u << left) - 1u;
-            }
-            uint32_t       ndeg  = 0;
+            uint32_t       ndeg  = 0, sel = 0;  // lane q: the chosen candidates of word q
             const uint32_t words = (m + 31u) / 32u;
             for (uint32_t k = 0; k < words && ndeg < R; ++k) {
-                uint32_t       wv  = __shfl_sync(0xffffffffu, live, k);
-                const uint32_t row = pm[(32u * k + lane) * QW + k];  // row t's bits within the word
-                uint32_t       got = 0u;
-                // p* = first live candidate; it and what it prunes leave the word
-                for (uint32_t room = R - ndeg; wv != 0u && room != 0u; --room) {
-                    const uint32_t t = __ffs(wv) - 1u;
-                    got |= 1u << t;
-                    wv &= ~(__shfl_sync(0xffffffffu, row, t) | (1u << t));
+                const uint32_t t   = 32u * k + lane;
+                uint32_t       out = t < m ? 0u : 1u;
+                for (uint32_t q = 0; q < k; ++q) {
+                    const uint32_t s = __shfl_sync(0xffffffffu, sel, q);
+                    out |= pby[q * MAXC + t] & s;
                 }
-                const bool mine = (got >> lane) & 1u;
-                if (mine) chosen[ndeg + __popc(got & ((1u << lane) - 1u))] = sid[32u * k + lane];
-                ndeg += __popc(got);
-                // the later words lose what the word's chosen candidates prune
-                for (uint32_t q = k + 1u; q < words; ++q) {
-                    const uint32_t out =
-                        __reduce_or_sync(0xffffffffu, mine ? pm[(32u * k + lane) * QW + q] : 0u);
-                    if (lane == q) live &= ~out;
+                const uint32_t by   = pby[k * MAXC + t] & ((1u << lane) - 1u);  // pruners within the word
+                uint32_t       und  = __ballot_sync(0xffffffffu, out == 0u);
+                uint32_t       got  = 0u;
+                while (und != 0u) {
+                    const bool     in  = (und >> lane) & 1u;
+                    const uint32_t now = __ballot_sync(0xffffffffu, in && (by & und) == 0u);
+                    got |= now;
+                    und &= ~now & ~__ballot_sync(0xffffffffu, in && (by & now) != 0u);
                 }
+                const uint32_t rank = __popc(got & ((1u << lane) - 1u));
+                const bool     mine = ((got >> lane) & 1u) && ndeg + rank < R;
+                if (mine) chosen[ndeg + rank] = sid[t] & ~kB;
+                ndeg = min(R, ndeg + __popc(got));
+                if (lane == k) sel = got;
             }
             if (lane == 0) {
                 misc[1]     = ndeg;
@@ -489,7 +492,7 @@ __global__ void __launch_bounds__(kThreads) prune_tc_kernel(PruneArgs a, uint32_
     __syncthreads();
     if (warp == 0) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols));
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(COLS));
     }
 }
 
@@ -499,7 +502,7 @@ bool prune_tc_supported(uint32_t D, uint32_t R) { return D % 32 == 0 && D >= 32 
 
 namespace {
 
-template <uint32_t MAXC>
+template <uint32_t MAXC, uint32_t COLS>
 cudaError_t launch_tc(const PruneArgs& a, uint32_t* counter, const uint32_t* in_list, const uint32_t* in_count,
                       uint32_t* out_list, uint32_t* out_count, uint64_t max_nodes, int num_sms, cudaStream_t st) {
     int dev = 0, per_sm_smem = 0, reserved = 0;
@@ -509,14 +512,14 @@ cudaError_t launch_tc(const PruneArgs& a, uint32_t* counter, const uint32_t* in_
     if (e != cudaSuccess) return e;
     e = cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev);
     if (e != cudaSuccess) return e;
-    // TMEM holds 512 columns per SM: at most 512 / kTmemCols CTAs of these kernels may
+    // TMEM holds 512 columns per SM: at most 512 / COLS CTAs of these kernels may
     // share an SM, which the shared-memory request enforces (an extra CTA would wait
     // in tcgen05.alloc for one of the others to exit).
-    const int    max_ctas    = 512 / (int)kTmemCols;
+    const int    max_ctas    = 512 / (int)COLS;
     size_t       smem        = TcLayout::make(a.D, MAXC).bytes;
     const size_t floor_bytes = (size_t)(per_sm_smem / (max_ctas + 1) - reserved + 1024);
     if (smem < floor_bytes) smem = floor_bytes;
-    auto kern = prune_tc_kernel<MAXC>;
+    auto kern = prune_tc_kernel<MAXC, COLS>;
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
@@ -535,11 +538,12 @@ cudaError_t launch_tc(const PruneArgs& a, uint32_t* counter, const uint32_t* in_
 
 }  // namespace
 
-// Passes of 256 candidates (4 CTAs per SM), then 512 (2 per SM), then 768 (one per
+// Passes of 128 candidates (up to 8 CTAs per SM), 256 (4), 512 (2), then 768 (one per
 // SM, when its shared memory fits: D <= 160), each over the nodes the previous one
 // handed on.  The first pass takes in_list[0 .. *in_count) (every node when null);
-// what the last cannot take goes to out_list for prune_kernel.
-// ws: 2 * n_nodes + 4 words of device scratch; counters: three zeroed work counters.
+// what the last cannot take goes to out_list for prune_kernel.  A launch of no more
+// nodes than SMs has nothing to fill with small passes: it goes straight to the last.
+// ws: 2 * n_nodes + 4 words of device scratch; counters: four zeroed work counters.
 cudaError_t launch_prune_tc(const PruneArgs& a, const uint32_t* in_list, const uint32_t* in_count,
                             uint32_t* out_list, uint32_t* out_count, uint32_t* ws, uint32_t* counters, int num_sms,
                             cudaStream_t st) {
@@ -551,20 +555,22 @@ cudaError_t launch_prune_tc(const PruneArgs& a, const uint32_t* in_list, const u
     if (e != cudaSuccess) return e;
     e = cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     if (e != cudaSuccess) return e;
-    const bool third  = TcLayout::make(a.D, 768).bytes <= (uint32_t)max_optin;
-    uint32_t*  list1  = ws;
-    uint32_t*  count1 = ws + a.n_nodes;
-    uint32_t*  list2  = third ? ws + a.n_nodes + 1 : out_list;
-    uint32_t*  count2 = third ? ws + 2 * a.n_nodes + 1 : out_count;
-    for (uint32_t* c : {count1, count2, out_count}) {
-        e = cudaMemsetAsync(c, 0, sizeof(uint32_t), st);
-        if (e != cudaSuccess) return e;
-    }
-    e = launch_tc<256>(a, counters, in_list, in_count, list1, count1, a.n_nodes, num_sms, st);
+    const bool last768 = TcLayout::make(a.D, 768).bytes <= (uint32_t)max_optin;
+    if ((e = cudaMemsetAsync(out_count, 0, sizeof(uint32_t), st)) != cudaSuccess) return e;
+    if (last768 && a.n_nodes <= (uint64_t)num_sms)
+        return launch_tc<768, 128>(a, counters, in_list, in_count, out_list, out_count, a.n_nodes, num_sms, st);
+    // the hand-off lists alternate between two halves of ws; their counts sit together
+    uint32_t* list[2] = {ws, ws + a.n_nodes};
+    uint32_t* cnt     = ws + 2 * a.n_nodes;  // one per hand-off
+    if ((e = cudaMemsetAsync(cnt, 0, 3 * sizeof(uint32_t), st)) != cudaSuccess) return e;
+    e = launch_tc<128, 64>(a, counters, in_list, in_count, list[0], cnt, a.n_nodes, num_sms, st);
     if (e != cudaSuccess) return e;
-    e = launch_tc<512>(a, counters + 1, list1, count1, list2, count2, a.n_nodes, num_sms, st);
-    if (e != cudaSuccess || !third) return e;
-    return launch_tc<768>(a, counters + 2, list2, count2, out_list, out_count, a.n_nodes, num_sms, st);
+    e = launch_tc<256, 128>(a, counters + 1, list[0], cnt, list[1], cnt + 1, a.n_nodes, num_sms, st);
+    if (e != cudaSuccess) return e;
+    if (!last768) return launch_tc<512, 128>(a, counters + 2, list[1], cnt + 1, out_list, out_count, a.n_nodes, num_sms, st);
+    e = launch_tc<512, 128>(a, counters + 2, list[1], cnt + 1, list[0], cnt + 2, a.n_nodes, num_sms, st);
+    if (e != cudaSuccess) return e;
+    return launch_tc<768, 128>(a, counters + 3, list[0], cnt + 2, out_list, out_count, a.n_nodes, num_sms, st);
 }
 
 }  // namespace vann
