@@ -260,7 +260,7 @@ __global__ void __launch_bounds__(kThreads, MAXC == 128 ? 8 : 1)
             cid[i] = id;
             cd[i]  = d;
         }
-        if (tid < 3u && nc + tid < MAXC)  // groups of four below read past an uneven count
+        if (tid < 32u && ((nc + 31u) & ~31u) > nc + tid)  // the last chunk of 32 is read whole below
             cd[nc + tid] = __uint_as_float(0xFFFFFFFFu);
         if (computed) {
             if (tid < nchunk)
@@ -289,7 +289,8 @@ __global__ void __launch_bounds__(kThreads, MAXC == 128 ? 8 : 1)
         __syncthreads();
 
         // --- 2. stable order by (distance, candidate index).  Distances are non-negative,
-        // so their bits order them; index i = 128 q + tid counts equal bits of lower index.
+        // so their bits order them: rank = distances below, plus equal ones of lower index
+        // (whole chunks of 32 by a raised bound, the candidate's own chunk by a match).
         const uint32_t m = min(nc, a.cap);
         {
             uint32_t b[KPT], r[KPT];
@@ -297,32 +298,22 @@ __global__ void __launch_bounds__(kThreads, MAXC == 128 ? 8 : 1)
             for (uint32_t q = 0; q < KPT; ++q) {
                 const uint32_t i = tid + q * kThreads;
                 b[q]             = i < nc ? __float_as_uint(cd[i]) : 0u;
-                r[q]             = 0;
+                r[q]             = __popc(__match_any_sync(0xffffffffu, b[q]) & ((1u << lane) - 1u));
             }
             const uint32_t used = (nc + kThreads - 1) / kThreads;  // candidates in use per thread
             for (uint32_t c0 = 0; c0 < nc; c0 += 32) {             // the warp's own chunk: 128 q + 32 warp
+                const uint4* dj = reinterpret_cast<const uint4*>(cd + c0);
+                uint32_t     thr[KPT];
 #pragma unroll
-                for (uint32_t q = 0; q < KPT; ++q) {
-                    if (q >= used) break;
-                    const uint32_t own = 128u * q + 32u * warp;
-                    const uint4*   dj  = reinterpret_cast<const uint4*>(cd + c0);
-                    const uint32_t n4  = min(8u, (nc - c0 + 3u) / 4u);
-                    if (c0 != own) {
-                        const uint32_t thr = b[q] + (c0 < own ? 1u : 0u);
-                        for (uint32_t j = 0; j < n4; ++j) {
-                            const uint4 x = dj[j];
-                            r[q] += (uint32_t)(x.x < thr) + (uint32_t)(x.y < thr) + (uint32_t)(x.z < thr) +
-                                    (uint32_t)(x.w < thr);
-                        }
-                    } else {
-                        for (uint32_t j = 0; j < n4; ++j) {
-                            const uint4 x = dj[j];
-                            r[q] += (uint32_t)(x.x < b[q] + (4u * j < lane ? 1u : 0u)) +
-                                    (uint32_t)(x.y < b[q] + (4u * j + 1u < lane ? 1u : 0u)) +
-                                    (uint32_t)(x.z < b[q] + (4u * j + 2u < lane ? 1u : 0u)) +
-                                    (uint32_t)(x.w < b[q] + (4u * j + 3u < lane ? 1u : 0u));
-                        }
-                    }
+                for (uint32_t q = 0; q < KPT; ++q) thr[q] = b[q] + (c0 < 128u * q + 32u * warp ? 1u : 0u);
+#pragma unroll
+                for (uint32_t j = 0; j < 8; ++j) {
+                    const uint4 x = dj[j];
+#pragma unroll
+                    for (uint32_t q = 0; q < KPT; ++q)
+                        if (q < used)
+                            r[q] += (uint32_t)(x.x < thr[q]) + (uint32_t)(x.y < thr[q]) + (uint32_t)(x.z < thr[q]) +
+                                    (uint32_t)(x.w < thr[q]);
                 }
             }
 #pragma unroll
@@ -382,6 +373,7 @@ __global__ void __launch_bounds__(kThreads, MAXC == 128 ? 8 : 1)
         __syncthreads();
 
         // --- 5. bits of the candidates that prune t
+        bool late = false;
         for (uint32_t r = 0; r < nb; ++r) {
             const uint32_t t = 128u * r + tid;
             // "u prunes t" is alpha * d(u, t) <= d(node, t) in FP32, with d(u, t) the exact
@@ -409,12 +401,8 @@ __global__ void __launch_bounds__(kThreads, MAXC == 128 ? 8 : 1)
                         issue_tile(r, c);
                     }
                 }
-                const bool ok = mbar_wait(bar, phase);
+                late |= !mbar_wait(bar, phase);
                 phase ^= 1u;
-                if (__syncthreads_or(!ok)) {
-                    failed = true;
-                    break;
-                }
                 tc_fence_after();
 #pragma unroll 1
                 for (uint32_t c32 = 0; c32 < COLS; c32 += 32u) {
@@ -440,11 +428,12 @@ __global__ void __launch_bounds__(kThreads, MAXC == 128 ? 8 : 1)
                     if (t < m) pby[(u0 >> 5) * MAXC + t] = word;
                 }
             }
-            if (failed) break;
         }
-        if (failed) break;
         tc_fence_before();
-        __syncthreads();
+        if (__syncthreads_or(late)) {  // a wait for the tensor cores gave up
+            failed = true;
+            break;
+        }
 
         // --- 6. selection (warp 0), a word of 32 candidates at a time
         if (warp == 0) {
