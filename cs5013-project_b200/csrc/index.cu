@@ -408,20 +408,21 @@ struct vann_index {
     }
 
     // RobustPrune launch.  Consistent reverse re-prunes go first to the warp-per-node
-    // kernel; the tensor-core passes take what it hands on (or every node) when an
-    // exact uint8 copy may exist (decided on the device by the exactness flag);
-    // prune_kernel finishes whatever is left.
+    // kernel; what it hands on (or every node) goes to the tensor-core passes, over the
+    // uint8 copy when it is exact, else over the FP32 rows where D allows; prune_kernel
+    // finishes whatever is left.
     void run_prune(vann::PruneArgs pa, cudaStream_t st) {
         if (pa.n_nodes == 0) return;
         pa.pruned = reinterpret_cast<unsigned long long*>(status + vann::kWordPruned);
         const uint64_t n   = pa.n_nodes;
-        const bool     tc  = store[3] && vann::prune_tc_supported(p.dim, p.degree);
+        const bool     tc  = vann::prune_tc_supported(p.dim, p.degree) && u8_exact(st);
+        const bool     f16 = !tc && vann::prune_f16_supported(p.dim, p.degree);
         const bool     rev = pa.consistent && pa.csr_off && pa.node_ids && p.dim <= 256;
         if (store[3]) {
             pa.vecs_u8 = static_cast<const uint8_t*>(store[3]);
             pa.gate    = u8_inexact();
         }
-        // lists: [0, n] rev hand-off + count, [n+1, 2n+2) final hand-off + count, then tc scratch
+        // lists: [0, n] rev hand-off + count, [n+1, 2n+2) final hand-off + count, then the passes' scratch
         ovf.ensure(sizeof(uint32_t) * (4 * n + 8));
         uint32_t*       rev_list   = ovf.as<uint32_t>();
         uint32_t*       rev_count  = rev_list + n;
@@ -442,6 +443,13 @@ struct vann_index {
             VCHECK(cudaMemsetAsync(tc_counters + 1, 0, 3 * sizeof(uint32_t), st));
             VCHECK(vann::launch_prune_tc(pa, in_list, in_count, last_list, last_count, ws, tc_counters, num_sms,
                                          st));
+            in_list  = last_list;
+            in_count = last_count;
+        } else if (f16) {
+            uint32_t* f16_counters = next_counter(st);  // one per pass
+            VCHECK(cudaMemsetAsync(f16_counters + 1, 0, 2 * sizeof(uint32_t), st));
+            VCHECK(vann::launch_prune_f16(pa, in_list, in_count, last_list, last_count, ws, f16_counters, num_sms,
+                                          st));
             in_list  = last_list;
             in_count = last_count;
         }

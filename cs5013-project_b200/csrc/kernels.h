@@ -99,6 +99,12 @@ bool        prune_tc_supported(uint32_t D, uint32_t R);
 cudaError_t launch_prune_tc(const PruneArgs& a, const uint32_t* in_list, const uint32_t* in_count,
                             uint32_t* out_list, uint32_t* out_count, uint32_t* ws, uint32_t* counters, int num_sms,
                             cudaStream_t st);
+// The same passes over float rows (D <= 128): a Gram matrix of f16 rows as a filter, pairs
+// it cannot decide by their FP32 distances.  ws as above; counters: three zeroed ones.
+bool        prune_f16_supported(uint32_t D, uint32_t R);
+cudaError_t launch_prune_f16(const PruneArgs& a, const uint32_t* in_list, const uint32_t* in_count,
+                             uint32_t* out_list, uint32_t* out_count, uint32_t* ws, uint32_t* counters, int num_sms,
+                             cudaStream_t st);
 // Reverse re-prune of consistent lists, one warp per node (prune_rev.cu): nodes
 // with more than 128 candidates or 8 reverse sources are handed on in out_list.
 // u8: distances from a.vecs_u8 (the host has read that every row is exact).

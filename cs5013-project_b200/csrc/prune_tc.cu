@@ -31,6 +31,20 @@
 // 768), larger ones to prune_kernel.  If the uint8 copy is not exact (a device flag
 // written by the conversion kernels) this kernel returns at once and prune_kernel does
 // all.
+//
+// Float rows (F16, D <= 128): the tensor cores are a filter, the decisions stay those of
+// FP32.  The rows are staged relative to the node, scaled by a power of two and rounded
+// to f16 (kind::f16, FP32 accumulators); a pair whose test is farther from equality than
+// the rounding can move it (a bound proven beside the test, 0.22% of d(node, t)) is
+// decided from the Gram entry.  The others, around 1% of the pairs, are listed and
+// decided by their FP32 distance, summed in the order the warp-per-node kernel sums it,
+// so every list has the bits prune_kernel gives.  A node with more undecided pairs than
+// the list holds goes to the next pass, at last to prune_kernel.  f16 and not tf32: the
+// same 11-bit significand (the scaling takes care of the range) at half the shared memory,
+// which is what limits the nodes in flight.  prune_kernel does a node's distances on the
+// CUDA cores from L2, 12 warps per SM: 42.2 ms of a 100k x 96 build's 58.7 ms.
+#include <cuda_fp16.h>
+
 #include "common.cuh"
 #include "kernels.h"
 
@@ -50,18 +64,27 @@ __device__ __forceinline__ uint64_t umma_desc(uint32_t addr, uint32_t lbo, uint3
            ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
 }
 
-// instruction descriptor: D s32, A and B unsigned 8-bit, both K-major
-__device__ __forceinline__ uint32_t idesc_u8(uint32_t M, uint32_t N) {
-    return (2u << 4) | ((N >> 3) << 17) | ((M >> 4) << 24);
+// instruction descriptor, A and B K-major and of one type: unsigned 8-bit into s32, or
+// f16 into f32
+template <bool F16>
+__device__ __forceinline__ uint32_t idesc(uint32_t M, uint32_t N) {
+    return ((F16 ? 1u : 2u) << 4) | ((N >> 3) << 17) | ((M >> 4) << 24);
 }
 
-__device__ __forceinline__ void mma_u8(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc,
-                                       uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem_d),
-        "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
-        : "memory");
+template <bool F16>
+__device__ __forceinline__ void mma(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t desc, uint32_t accumulate) {
+    if constexpr (F16)
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem_d),
+            "l"(da), "l"(db), "r"(desc), "r"(accumulate)
+            : "memory");
+    else
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem_d),
+            "l"(da), "l"(db), "r"(desc), "r"(accumulate)
+            : "memory");
 }
 
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
@@ -117,49 +140,81 @@ __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.
 
 __device__ __forceinline__ uint32_t dp4a_u(uint32_t a, uint32_t b, uint32_t c) { return __dp4a(a, b, c); }
 
+// Bytes of a staged row: D uint8, or D f16 padded to the MMA's K of 16.
+__host__ __device__ constexpr uint32_t staged_bytes(uint32_t D, bool f16) {
+    return f16 ? 2u * ((D + 15u) & ~15u) : D;
+}
+
 // shared memory of one CTA handling up to maxc candidates per node
 struct TcLayout {
-    uint32_t rows, nodev, cid, cd, sid, sd, nrm, pby, bmask, chosen, bar, misc, bytes;
-    __host__ __device__ static TcLayout make(uint32_t D, uint32_t maxc) {
+    uint32_t rows, nodev, cid, cd, sid, sd, nrm, pby, bmask, chosen, pairs, bar, misc, bytes;
+    __host__ __device__ static TcLayout make(uint32_t D, uint32_t maxc, bool f16) {
         TcLayout l;
-        l.rows   = 0;                  // maxc x D bytes, canonical layout, sorted order
-        l.nodev  = l.rows + maxc * D;  // D bytes
-        l.cid    = l.nodev + ((D + 15) & ~15u);
+        l.rows   = 0;  // maxc staged rows, canonical layout, sorted order
+        l.nodev  = l.rows + maxc * staged_bytes(D, f16);  // the node's row: uint8 or FP32
+        l.cid    = l.nodev + ((f16 ? 4u * D : D) + 15u & ~15u);
         l.cd     = l.cid + 4 * maxc;  // candidate order (A then B)
         l.sid    = l.cd + 4 * maxc;   // sorted order: id (top bit: a B candidate), distance,
-        l.sd     = l.sid + 4 * maxc;  // squared norm
+        l.sd     = l.sid + 4 * maxc;  // squared norm (uint8 rows)
         l.nrm    = l.sd + 4 * maxc;
-        l.pby    = l.nrm + 4 * maxc;  // [maxc / 32][maxc] bits of the candidates that prune t
-        l.bmask  = l.pby + maxc * maxc / 8;  // sorted positions holding B candidates
-        l.chosen = l.bmask + maxc / 8;       // the node's new list
-        l.bar    = l.chosen + 4 * kMaxR;
+        l.pby    = l.nrm + (f16 ? 0u : 4 * maxc);  // [maxc / 32][maxc] bits of the candidates that prune t
+        l.bmask  = l.pby + maxc * maxc / 8;        // sorted positions holding B candidates
+        l.chosen = l.bmask + 16 * ((maxc + kThreads - 1) / kThreads);  // the node's new list
+        l.pairs  = l.chosen + 4 * kMaxR;                               // undecided pairs (f16 rows)
+        l.bar    = l.pairs + (f16 ? 4 * kPairs(maxc) : 0u);
         l.misc   = l.bar + 8;
         l.bytes  = l.misc + 4 * 16;
         return l;
     }
+    // undecided pairs a node may have; one with more goes to the next pass
+    __host__ __device__ static constexpr uint32_t kPairs(uint32_t maxc) { return maxc > 512u ? 2048u : 4u * maxc; }
 };
+
+// FP32 squared distance of rows x and y by a half warp (lane t of 16), in the order of
+// dist_group<StoreF32> in the D <= 128 class: 8 dimensions per lane, even and odd
+// apart, then the lanes pairwise (^ 8, 4, 2, 1).
+__device__ __forceinline__ float half_warp_dist(const float* x, const float* y, uint32_t D, uint32_t t) {
+    const float2 neg1 = make_float2(-1.f, -1.f);
+    float2       acc  = make_float2(0.f, 0.f);
+#pragma unroll
+    for (uint32_t c = 0; c < 2; ++c) {
+        const uint32_t d0 = 8u * t + 4u * c;
+        if (d0 < D) {
+            const float4 a = __ldg(reinterpret_cast<const float4*>(x + d0));
+            const float4 b = __ldg(reinterpret_cast<const float4*>(y + d0));
+            float2       d = __ffma2_rn(make_float2(a.x, a.y), neg1, make_float2(b.x, b.y));
+            acc            = __ffma2_rn(d, d, acc);
+            d              = __ffma2_rn(make_float2(a.z, a.w), neg1, make_float2(b.z, b.w));
+            acc            = __ffma2_rn(d, d, acc);
+        }
+    }
+    float v = acc.x + acc.y;
+#pragma unroll
+    for (int o = 8; o >= 1; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
 
 // Nodes are the slots in_list[0 .. *in_count) (or 0 .. n_nodes when in_list is
 // null); nodes with more than MAXC candidates go to out_list.  COLS: TMEM columns per
-// CTA, the width of a Gram tile.
-template <uint32_t MAXC, uint32_t COLS>
+// CTA, the width of a Gram tile.  F16: float rows (the filter described above).
+template <uint32_t MAXC, uint32_t COLS, bool F16>
 __global__ void __launch_bounds__(kThreads, MAXC == 128 ? 8 : 1)
     prune_tc_kernel(PruneArgs a, uint32_t* counter, const uint32_t* in_list, const uint32_t* in_count,
                     uint32_t* out_list, uint32_t* out_count) {
-    constexpr uint32_t KPT = MAXC / kThreads;  // candidates per thread
+    constexpr uint32_t KPT = (MAXC + kThreads - 1) / kThreads;  // candidates per thread
     constexpr uint32_t kB  = 0x80000000u;      // sid: a B candidate (ids are below 2^31)
     extern __shared__ __align__(1024) unsigned char smem[];
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     const uint64_t nwork = in_list ? (uint64_t)*reinterpret_cast<volatile const uint32_t*>(in_count) : a.n_nodes;
     if (nwork == 0) return;
-    if (*reinterpret_cast<volatile const uint32_t*>(a.gate) != 0u) {  // rows not exact: hand every node on
+    if (!F16 && *reinterpret_cast<volatile const uint32_t*>(a.gate) != 0u) {  // rows not exact: hand every node on
         for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + tid; i < nwork; i += (uint64_t)gridDim.x * blockDim.x)
             out_list[atomicAdd(out_count, 1u)] = in_list ? __ldg(in_list + i) : (uint32_t)i;
         return;
     }
 
     const uint32_t D = a.D, R = a.R;
-    const TcLayout lay = TcLayout::make(D, MAXC);
+    const TcLayout lay = TcLayout::make(D, MAXC, F16);
     unsigned char* rows   = smem + lay.rows;
     uint8_t*       nodev  = smem + lay.nodev;
     uint32_t*      cid    = reinterpret_cast<uint32_t*>(smem + lay.cid);
@@ -170,7 +225,9 @@ __global__ void __launch_bounds__(kThreads, MAXC == 128 ? 8 : 1)
     uint32_t*      pby    = reinterpret_cast<uint32_t*>(smem + lay.pby);
     uint32_t*      bmask  = reinterpret_cast<uint32_t*>(smem + lay.bmask);
     uint32_t*      chosen = reinterpret_cast<uint32_t*>(smem + lay.chosen);
-    uint32_t*      misc   = reinterpret_cast<uint32_t*>(smem + lay.misc);  // [0] tmem, [1] degree, [2..13] work items
+    uint32_t*      pairs  = reinterpret_cast<uint32_t*>(smem + lay.pairs);
+    // [0] tmem, [1] degree, [2..13] work items, [14] undecided pairs
+    uint32_t*      misc   = reinterpret_cast<uint32_t*>(smem + lay.misc);
     const uint32_t bar    = saddr(smem + lay.bar);
     const uint32_t rows_s = saddr(rows);
 
@@ -189,10 +246,11 @@ __global__ void __launch_bounds__(kThreads, MAXC == 128 ? 8 : 1)
     const uint32_t tmem = misc[0];
 
     const bool     rev    = a.csr_off != nullptr;
-    const uint32_t nchunk = D / 16;
+    const uint32_t RB     = staged_bytes(D, F16);
+    const uint32_t nchunk = RB / 16;  // 16-byte chunks of a staged row
     const uint32_t inv_nc = 0xFFFFFFFFu / nchunk + 1u;  // x / nchunk = __umulhi(x, inv_nc), nchunk >= 2
-    const uint32_t LBO = 128, SBO = 8 * D;  // 8 rows x 16 B per core matrix; chunks adjacent
-    const uint32_t ksteps = D / 32;         // kind::i8: K = 32 per instruction
+    const uint32_t LBO = 128, SBO = 8 * RB;  // 8 rows x 16 B per core matrix; chunks adjacent
+    const uint32_t ksteps = RB / 32;        // K = 32 (kind::i8) or 16 (kind::f16) per instruction
     uint32_t       phase  = 0;
     bool           failed = false;
     uint32_t       done   = 0;  // nodes pruned by this CTA
@@ -262,7 +320,21 @@ __global__ void __launch_bounds__(kThreads, MAXC == 128 ? 8 : 1)
         }
         if (tid < 32u && ((nc + 31u) & ~31u) > nc + tid)  // the last chunk of 32 is read whole below
             cd[nc + tid] = __uint_as_float(0xFFFFFFFFu);
-        if (computed) {
+        if constexpr (F16) {
+            if (tid < D / 4u)
+                reinterpret_cast<float4*>(nodev)[tid] =
+                    __ldg(reinterpret_cast<const float4*>(a.vecs + (uint64_t)node * D) + tid);
+            const uint32_t first = (rev || a.a_d == nullptr) ? 0u : nA;
+            if (first < nc) {  // missing distances from the FP32 rows, as the search takes them
+                constexpr uint32_t G = Layout<StoreF32, 0>::kG;
+                __syncthreads();
+                Query<StoreF32, 0> nv;
+                load_query<StoreF32, 0>(nv, a.vecs + (uint64_t)node * D, D, lane);
+                for (uint32_t g0 = first + warp * G; g0 < nc; g0 += G * (kThreads / 32u))
+                    dist_round<StoreF32, 0>(nv, a.vecs, nullptr, [&](int j) { return cid[g0 + j]; },
+                                            (int)min(G, nc - g0), D, lane, cd + g0);
+            }
+        } else if (computed) {
             if (tid < nchunk)
                 *reinterpret_cast<uint4*>(nodev + 16 * tid) =
                     __ldg(reinterpret_cast<const uint4*>(a.vecs_u8 + (uint64_t)node * D) + tid);
@@ -328,10 +400,44 @@ __global__ void __launch_bounds__(kThreads, MAXC == 128 ? 8 : 1)
         __syncthreads();
 
         // --- 3. the first `cap` candidates' rows staged for the MMA
-        for (uint32_t x = tid; x < m * nchunk; x += kThreads) {
-            const uint32_t t = __umulhi(x, inv_nc), c = x - t * nchunk;
-            cp_async16(rows_s + (t >> 3) * SBO + c * LBO + (t & 7u) * 16u,
-                       a.vecs_u8 + (uint64_t)(sid[t] & ~kB) * D + 16u * c);
+        float g2 = 0.f, slack = 0.f;  // f16 rows: 2 / scale^2, and the error bound's constant part
+        if constexpr (F16) {
+            // rows relative to the node, scaled by a power of two so that the longest is
+            // at most 2^14, rounded to f16
+            const float smax = m > 0u ? sd[m - 1u] : 0.f;  // squared length of the longest
+            const bool  sane = smax > 1e-30f && smax < 1e37f;
+            int         e    = 0;
+            if (sane) frexpf(smax, &e);  // smax < 2^e
+            const int   h    = 14 - ((e + 1) >> 1);
+            const float up   = ldexpf(1.f, h);
+            g2               = ldexpf(2.f, -2 * h);
+            slack            = sane ? 1e-9f * smax : __int_as_float(0x7f800000);
+            const float4* nf = reinterpret_cast<const float4*>(nodev);
+            if (tid == 0) misc[14] = 0u;
+#pragma unroll 4
+            for (uint32_t x = tid; x < m * nchunk; x += kThreads) {
+                const uint32_t t = __umulhi(x, inv_nc), c = x - t * nchunk;
+                const float4*  src = reinterpret_cast<const float4*>(a.vecs + (uint64_t)(sid[t] & ~kB) * D) + 2u * c;
+                uint32_t       p[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+                for (uint32_t v = 0; v < 2; ++v) {
+                    if (8u * c + 4u * v < D) {
+                        const float4  r = __ldg(src + v), n = nf[2u * c + v];
+                        const __half2 lo = __floats2half2_rn((r.x - n.x) * up, (r.y - n.y) * up);
+                        const __half2 hi = __floats2half2_rn((r.z - n.z) * up, (r.w - n.w) * up);
+                        p[2 * v]         = *reinterpret_cast<const uint32_t*>(&lo);
+                        p[2 * v + 1]     = *reinterpret_cast<const uint32_t*>(&hi);
+                    }
+                }
+                *reinterpret_cast<uint4*>(rows + (t >> 3) * SBO + c * LBO + (t & 7u) * 16u) =
+                    make_uint4(p[0], p[1], p[2], p[3]);
+            }
+        } else {
+            for (uint32_t x = tid; x < m * nchunk; x += kThreads) {
+                const uint32_t t = __umulhi(x, inv_nc), c = x - t * nchunk;
+                cp_async16(rows_s + (t >> 3) * SBO + c * LBO + (t & 7u) * 16u,
+                           a.vecs_u8 + (uint64_t)(sid[t] & ~kB) * D + 16u * c);
+            }
         }
         if (a.consistent) {
 #pragma unroll
@@ -350,11 +456,11 @@ __global__ void __launch_bounds__(kThreads, MAXC == 128 ? 8 : 1)
         auto issue_tile = [&](uint32_t r, uint32_t c) {
             const uint32_t left = m - COLS * c;
             const uint32_t N    = ((left < COLS ? left : COLS) + 15u) & ~15u;
-            const uint32_t id   = idesc_u8(128u, N);
+            const uint32_t id   = idesc<F16>(128u, N);
             for (uint32_t s = 0; s < ksteps; ++s) {
                 const uint64_t da = umma_desc(rows_s + r * 16u * SBO + s * 2u * LBO, LBO, SBO);
                 const uint64_t db = umma_desc(rows_s + c * (COLS / 8u) * SBO + s * 2u * LBO, LBO, SBO);
-                mma_u8(tmem, da, db, id, s > 0 ? 1u : 0u);
+                mma<F16>(tmem, da, db, id, s > 0 ? 1u : 0u);
             }
             mma_commit(bar);
         };
@@ -362,15 +468,17 @@ __global__ void __launch_bounds__(kThreads, MAXC == 128 ? 8 : 1)
             tc_fence_after();
             issue_tile(0, 0);
         }
-        for (uint32_t t = tid; t < m; t += kThreads) {
-            uint32_t n = 0;
-            for (uint32_t c = 0; c < nchunk; ++c) {
-                const uint4 v = *reinterpret_cast<const uint4*>(rows + (t >> 3) * SBO + c * LBO + (t & 7u) * 16u);
-                n = dp4a_u(v.x, v.x, dp4a_u(v.y, v.y, dp4a_u(v.z, v.z, dp4a_u(v.w, v.w, n))));
+        if constexpr (!F16) {
+            for (uint32_t t = tid; t < m; t += kThreads) {
+                uint32_t n = 0;
+                for (uint32_t c = 0; c < nchunk; ++c) {
+                    const uint4 v = *reinterpret_cast<const uint4*>(rows + (t >> 3) * SBO + c * LBO + (t & 7u) * 16u);
+                    n = dp4a_u(v.x, v.x, dp4a_u(v.y, v.y, dp4a_u(v.z, v.z, dp4a_u(v.w, v.w, n))));
+                }
+                nrm[t] = n;
             }
-            nrm[t] = n;
+            __syncthreads();
         }
-        __syncthreads();
 
         // --- 5. bits of the candidates that prune t
         bool late = false;
@@ -380,14 +488,29 @@ __global__ void __launch_bounds__(kThreads, MAXC == 128 ? 8 : 1)
             // integer Y = |u|^2 + |t|^2 - 2 u.t (< 2^24, so FP32 holds it exactly).  fl(Y *
             // alpha) does not decrease as Y grows, so the test is Y <= Ymax(t), the largest
             // integer with fl(Ymax * alpha) <= d(node, t): 2 u.t - |u|^2 >= |t|^2 - Ymax(t).
+            // Float rows: with the Gram entry g of the f16 rows, d(u, t) is su + st - g2 g up
+            // to an error E, so u prunes t for certain where g2 g - su > st - st / alpha + E,
+            // and for certain not where it is < st - st / alpha - E (su <= st: u comes first).
+            // E: f16 rounding of both rows (2^-11 of each component) and the tensor core's
+            // FP32 accumulation, 2 (2^-10 + 2^-15) sqrt(su st) <= 0.00202 st; the FP32 sums
+            // su, st and d(u, t) themselves and this test's arithmetic, 4e-5 st; f16
+            // subnormals, 1e-9 of the longest row; FP32 subnormals, 1e-37.
             int      thr  = 0;
+            float    flo = 0.f, fhi = 0.f;
             uint32_t keep = ~0u;  // consistent lists: no B candidate is checked against another
             if (t < m) {
                 const float sdt = sd[t];
-                int         y   = (int)fminf(floorf(sdt / a.alpha), 16777215.f);
-                while (y < 16777215 && (float)(y + 1) * a.alpha <= sdt) ++y;
-                while (y > 0 && (float)y * a.alpha > sdt) --y;
-                thr = (int)nrm[t] - y;
+                if constexpr (F16) {
+                    const float mid = sdt - sdt / a.alpha;
+                    const float err = 0.0022f * sdt + slack + 1e-37f;
+                    flo             = mid - err;
+                    fhi             = mid + err;
+                } else {
+                    int y = (int)fminf(floorf(sdt / a.alpha), 16777215.f);
+                    while (y < 16777215 && (float)(y + 1) * a.alpha <= sdt) ++y;
+                    while (y > 0 && (float)y * a.alpha > sdt) --y;
+                    thr = (int)nrm[t] - y;
+                }
                 if (a.consistent && (sid[t] & kB)) keep = 0u;
             }
             const uint32_t last  = 128u * r + 32u * warp + 31u;  // the warp's last candidate
@@ -408,7 +531,7 @@ __global__ void __launch_bounds__(kThreads, MAXC == 128 ? 8 : 1)
                 for (uint32_t c32 = 0; c32 < COLS; c32 += 32u) {
                     const uint32_t u0 = COLS * c + c32;
                     if (u0 >= m || u0 > last) break;
-                    uint32_t word = 0;
+                    uint32_t word = 0, open = 0;  // open: undecided (float rows)
 #pragma unroll
                     for (uint32_t h = 0; h < 32u; h += 16u) {
                         if (u0 + h < m) {
@@ -416,16 +539,39 @@ __global__ void __launch_bounds__(kThreads, MAXC == 128 ? 8 : 1)
                             tmem_ld16(tmem + ((32u * warp) << 16) + c32 + h, g);
 #pragma unroll
                             for (uint32_t k = 0; k < 16; k += 4) {
-                                const uint4 nu = *reinterpret_cast<const uint4*>(nrm + u0 + h + k);
-                                word |= (uint32_t)((int)(2u * g[k] - nu.x) >= thr) << (h + k);
-                                word |= (uint32_t)((int)(2u * g[k + 1] - nu.y) >= thr) << (h + k + 1);
-                                word |= (uint32_t)((int)(2u * g[k + 2] - nu.z) >= thr) << (h + k + 2);
-                                word |= (uint32_t)((int)(2u * g[k + 3] - nu.w) >= thr) << (h + k + 3);
+                                if constexpr (F16) {
+                                    const float4 su  = *reinterpret_cast<const float4*>(sd + u0 + h + k);
+                                    const float  x[4] = {fmaf(__uint_as_float(g[k]), g2, -su.x),
+                                                         fmaf(__uint_as_float(g[k + 1]), g2, -su.y),
+                                                         fmaf(__uint_as_float(g[k + 2]), g2, -su.z),
+                                                         fmaf(__uint_as_float(g[k + 3]), g2, -su.w)};
+#pragma unroll
+                                    for (uint32_t i = 0; i < 4; ++i) {
+                                        const bool yes = x[i] > fhi;
+                                        word |= (uint32_t)yes << (h + k + i);
+                                        open |= (uint32_t)(!yes && !(x[i] < flo)) << (h + k + i);
+                                    }
+                                } else {
+                                    const uint4 nu = *reinterpret_cast<const uint4*>(nrm + u0 + h + k);
+                                    word |= (uint32_t)((int)(2u * g[k] - nu.x) >= thr) << (h + k);
+                                    word |= (uint32_t)((int)(2u * g[k + 1] - nu.y) >= thr) << (h + k + 1);
+                                    word |= (uint32_t)((int)(2u * g[k + 2] - nu.z) >= thr) << (h + k + 2);
+                                    word |= (uint32_t)((int)(2u * g[k + 3] - nu.w) >= thr) << (h + k + 3);
+                                }
                             }
                         }
                     }
                     if (keep == 0u) word &= ~bmask[u0 >> 5];
                     if (t < m) pby[(u0 >> 5) * MAXC + t] = word;
+                    if constexpr (F16) {
+                        if (keep == 0u) open &= ~bmask[u0 >> 5];
+                        if (u0 + 32u > t) open &= t > u0 ? (1u << (t - u0)) - 1u : 0u;  // earlier candidates only
+                        if (t < m && open != 0u) {
+                            uint32_t at = atomicAdd(&misc[14], __popc(open));
+                            for (; open != 0u && at < TcLayout::kPairs(MAXC); open &= open - 1u, ++at)
+                                pairs[at] = (t << 16) | (u0 + __ffs(open) - 1u);
+                        }
+                    }
                 }
             }
         }
@@ -433,6 +579,24 @@ __global__ void __launch_bounds__(kThreads, MAXC == 128 ? 8 : 1)
         if (__syncthreads_or(late)) {  // a wait for the tensor cores gave up
             failed = true;
             break;
+        }
+
+        if constexpr (F16) {
+            // undecided pairs by their FP32 distance, a half warp each
+            const uint32_t np = misc[14];
+            if (np > TcLayout::kPairs(MAXC)) {
+                if (tid == 0) out_list[atomicAdd(out_count, 1u)] = w;
+                continue;
+            }
+            for (uint32_t p0 = 2u * warp; p0 < np; p0 += 2u * (kThreads / 32u)) {
+                const uint32_t p  = p0 + (lane >> 4);
+                const uint32_t pr = pairs[min(p, np - 1u)], t = pr >> 16, u = pr & 0xffffu;
+                const float    y  = half_warp_dist(a.vecs + (uint64_t)(sid[u] & ~kB) * D,
+                                                   a.vecs + (uint64_t)(sid[t] & ~kB) * D, D, lane & 15u);
+                if ((lane & 15u) == 0u && p < np && y * a.alpha <= sd[t])
+                    atomicOr(&pby[(u >> 5) * MAXC + t], 1u << (u & 31u));
+            }
+            __syncthreads();
         }
 
         // --- 6. selection (warp 0), a word of 32 candidates at a time
@@ -476,7 +640,7 @@ __global__ void __launch_bounds__(kThreads, MAXC == 128 ? 8 : 1)
         ++done;
     }
     if (failed && tid == 0) atomicOr(a.status, kStatusTimeout);
-    if (tid == 0 && a.pruned && done) atomicAdd(a.pruned, (unsigned long long)done);
+    if (tid == 0 && a.pruned && done) atomicAdd(a.pruned + (F16 ? 1 : 0), (unsigned long long)done);
     tc_fence_before();
     __syncthreads();
     if (warp == 0) {
@@ -488,10 +652,11 @@ __global__ void __launch_bounds__(kThreads, MAXC == 128 ? 8 : 1)
 }  // namespace
 
 bool prune_tc_supported(uint32_t D, uint32_t R) { return D % 32 == 0 && D >= 32 && D <= 256 && R <= kMaxR; }
+bool prune_f16_supported(uint32_t D, uint32_t R) { return D <= 128 && R <= kMaxR; }
 
 namespace {
 
-template <uint32_t MAXC, uint32_t COLS>
+template <uint32_t MAXC, uint32_t COLS, bool F16 = false>
 cudaError_t launch_tc(const PruneArgs& a, uint32_t* counter, const uint32_t* in_list, const uint32_t* in_count,
                       uint32_t* out_list, uint32_t* out_count, uint64_t max_nodes, int num_sms, cudaStream_t st) {
     int dev = 0, per_sm_smem = 0, reserved = 0;
@@ -505,10 +670,10 @@ cudaError_t launch_tc(const PruneArgs& a, uint32_t* counter, const uint32_t* in_
     // share an SM, which the shared-memory request enforces (an extra CTA would wait
     // in tcgen05.alloc for one of the others to exit).
     const int    max_ctas    = 512 / (int)COLS;
-    size_t       smem        = TcLayout::make(a.D, MAXC).bytes;
+    size_t       smem        = TcLayout::make(a.D, MAXC, F16).bytes;
     const size_t floor_bytes = (size_t)(per_sm_smem / (max_ctas + 1) - reserved + 1024);
     if (smem < floor_bytes) smem = floor_bytes;
-    auto kern = prune_tc_kernel<MAXC, COLS>;
+    auto kern = prune_tc_kernel<MAXC, COLS, F16>;
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
@@ -544,7 +709,7 @@ cudaError_t launch_prune_tc(const PruneArgs& a, const uint32_t* in_list, const u
     if (e != cudaSuccess) return e;
     e = cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     if (e != cudaSuccess) return e;
-    const bool last768 = TcLayout::make(a.D, 768).bytes <= (uint32_t)max_optin;
+    const bool last768 = TcLayout::make(a.D, 768, false).bytes <= (uint32_t)max_optin;
     if ((e = cudaMemsetAsync(out_count, 0, sizeof(uint32_t), st)) != cudaSuccess) return e;
     if (last768 && a.n_nodes <= (uint64_t)num_sms)
         return launch_tc<768, 128>(a, counters, in_list, in_count, out_list, out_count, a.n_nodes, num_sms, st);
@@ -560,6 +725,26 @@ cudaError_t launch_prune_tc(const PruneArgs& a, const uint32_t* in_list, const u
     e = launch_tc<512, 128>(a, counters + 2, list[1], cnt + 1, list[0], cnt + 2, a.n_nodes, num_sms, st);
     if (e != cudaSuccess) return e;
     return launch_tc<768, 128>(a, counters + 3, list[0], cnt + 2, out_list, out_count, a.n_nodes, num_sms, st);
+}
+
+// The same over float rows: passes of 128, 256 and 576 candidates.  ws: 2 * n_nodes + 2
+// words of device scratch; counters: three zeroed work counters.
+cudaError_t launch_prune_f16(const PruneArgs& a, const uint32_t* in_list, const uint32_t* in_count,
+                             uint32_t* out_list, uint32_t* out_count, uint32_t* ws, uint32_t* counters, int num_sms,
+                             cudaStream_t st) {
+    if (a.n_nodes == 0) return cudaSuccess;
+    if (!prune_f16_supported(a.D, a.R) || !out_list || !out_count) return cudaErrorInvalidValue;
+    cudaError_t e = cudaMemsetAsync(out_count, 0, sizeof(uint32_t), st);
+    if (e != cudaSuccess) return e;
+    if (a.n_nodes <= (uint64_t)num_sms)
+        return launch_tc<576, 128, true>(a, counters, in_list, in_count, out_list, out_count, a.n_nodes, num_sms, st);
+    uint32_t *list1 = ws, *list2 = ws + a.n_nodes, *cnt = ws + 2 * a.n_nodes;
+    if ((e = cudaMemsetAsync(cnt, 0, 2 * sizeof(uint32_t), st)) != cudaSuccess) return e;
+    e = launch_tc<128, 64, true>(a, counters, in_list, in_count, list1, cnt, a.n_nodes, num_sms, st);
+    if (e != cudaSuccess) return e;
+    e = launch_tc<256, 128, true>(a, counters + 1, list1, cnt, list2, cnt + 1, a.n_nodes, num_sms, st);
+    if (e != cudaSuccess) return e;
+    return launch_tc<576, 128, true>(a, counters + 2, list2, cnt + 1, out_list, out_count, a.n_nodes, num_sms, st);
 }
 
 }  // namespace vann
