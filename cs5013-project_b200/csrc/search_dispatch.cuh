@@ -1,8 +1,10 @@
 // search_dispatch.cuh -- picks the search kernel instantiation for a launch:
 // register worklist (search_reg.cuh) for L <= 64 at D <= 128 and R <= 64,
-// shared-memory worklist (search_impl.cuh) otherwise, and the launch-bound
+// shared-memory worklist (search_impl.cuh) otherwise, a CTA per query (search_cta.cuh)
+// for small batches of either, and the launch-bound
 // variant chosen by the autotuner.
 #pragma once
+#include "search_cta.cuh"
 #include "search_reg.cuh"
 
 namespace vann {
@@ -70,9 +72,35 @@ static cudaError_t launch_r(const SearchArgs& a, int variant, int sms, cudaStrea
     return launch_v<S, DC, 4>(a, variant, sms, st);
 }
 
+// Batches served by a CTA per query (search_cta.cuh): up to as many queries as keep it
+// ahead of a warp per query, which needs many to fill the chip but then does more of them.
+// Measured on 148 SMs, CTA / warp per query in us (10 to 1,500 queries):
+//   worklist in registers otherwise (L <= 64): uint8 1M x 128, L = 64: 1 query 92 / 114,
+//     300 queries 254 / 305, 590 320 / 373, 900 400 / 415, 1,500 509 / 422; uint8 L = 32: 590
+//     118 / 134, 700 148 / 135;
+//   L <= 128, or wider rows or lists: FP32 200k x 96, L = 100: 1 query 125 / 211, 590 300 /
+//     479, 1,000 371 / 481, 1,200 494 / 476; BF16 100k x 256, L = 128 with rerank: 1 query
+//     241 / 493, 1,000 976 / 1,074, 1,200 1,126 / 1,110;
+//   L <= 256 (more registers, fewer CTAs): FP32 L = 200: 1 query 194 / 319, 300 248 / 416, 590
+//     451 / 429.
+inline bool small_batch(const SearchArgs& a, int sms) {
+    if (a.beam == 2 || a.L > kCtaMaxL) return false;
+    const uint64_t per_sm = a.L > 128 ? 3 : (a.L > 64 || a.D > 128 || a.R > 64 ? 7 : 4);
+    return a.nq <= per_sm * (uint64_t)sms;
+}
+
 template <typename S>
 static cudaError_t launch_store(const SearchArgs& a, int variant, int sms, cudaStream_t st) {
     if (a.D % S::kElems != 0) return cudaErrorInvalidValue;
+    if constexpr (!S::kPQ) {
+        if (small_batch(a, sms)) {
+            if constexpr (S::kInt)
+                if (a.int_queries && a.D <= 128) return launch_cta<S, 0, true>(a, sms, st);
+            if (a.D <= 128) return launch_cta<S, 0>(a, sms, st);
+            if (a.D <= 256) return launch_cta<S, 1>(a, sms, st);
+            return launch_cta<S, 2>(a, sms, st);
+        }
+    }
     if (a.D <= 128) return launch_r<S, 0>(a, variant, sms, st);
     if (a.D <= 256) return launch_r<S, 1>(a, variant, sms, st);
     return launch_r<S, 2>(a, variant, sms, st);
