@@ -318,16 +318,17 @@ __device__ __forceinline__ V group_reduce(V (&v)[M], uint32_t lane) {
 
 // Row (within a gather round) whose distance lane `lane` holds after dist_group,
 // and whether this lane is the one that writes it.
-template <typename S, int DC>
+// M: rows per lane per round (a power of two up to the layout's).
+template <typename S, int DC, int M = Layout<S, DC>::kM>
 __device__ __forceinline__ uint32_t round_row_of_lane(uint32_t lane) {
     using Ly        = Layout<S, DC>;
     const uint32_t t = lane % Ly::kT, g = lane / Ly::kT;
-    return (t / (Ly::kT / Ly::kM)) * Ly::kP + g;
+    return (t / (Ly::kT / M)) * Ly::kP + g;
 }
-template <typename S, int DC>
+template <typename S, int DC, int M = Layout<S, DC>::kM>
 __device__ __forceinline__ bool round_writer(uint32_t lane) {
     using Ly = Layout<S, DC>;
-    return (lane % (Ly::kT / Ly::kM)) == 0u;
+    return (lane % (Ly::kT / M)) == 0u;
 }
 
 // Squared L2 from the query to rows ids(0) .. ids(cnt-1), cnt <= kG (uniform
@@ -340,11 +341,13 @@ __device__ __forceinline__ bool round_writer(uint32_t lane) {
 // kIntQuery (integer stores): the caller knows the query is integer-valued (a row of
 // an exact uint8 copy), so the FP32 fallback for other queries is not compiled in;
 // its registers would otherwise set the kernel's count.
-template <typename S, int DC, bool kIntQuery = false, typename IdFn>
+//
+// M: rows per lane (rounds of M * kP rows); a row's sum is taken in the same order for
+// every M.
+template <typename S, int DC, bool kIntQuery = false, int M = Layout<S, DC>::kM, typename IdFn>
 __device__ __forceinline__ float dist_group(const Query<S, DC>& q, const void* base, const float2* scale,
                                             IdFn ids, int cnt, uint32_t D, uint32_t lane) {
     using Ly                 = Layout<S, DC>;
-    constexpr int  M         = Ly::kM;
     const uint32_t chunks    = D / S::kElems;
     const uint64_t row_bytes = (uint64_t)D * 16u / (uint64_t)S::kElems;
     const uint32_t t         = lane % Ly::kT;

@@ -46,6 +46,17 @@ struct CtaSearchLayout {
     }
 };
 
+// Rows per lane in a gather round here: a hop measures some 6 to 30 rows, a quarter of
+// them per warp, so rounds of 4 (FP32) to 8 rows, where the warp-per-query kernels take 8
+// to 32; fewer registers, more CTAs per SM, no arithmetic for rows that are not there.
+template <typename S, int DC>
+struct CtaRows {
+    static constexpr int kWant = S::kInt ? 8 : 4;  // rows per round
+    static constexpr int kP    = Layout<S, DC>::kP;
+    static constexpr int kFit  = kWant >= kP ? kWant / kP : 1;
+    static constexpr int kM    = kFit < Layout<S, DC>::kM ? kFit : Layout<S, DC>::kM;
+};
+
 // warps 1-4
 __device__ __forceinline__ void gather_barrier() {
     asm volatile("bar.sync 1, %0;" ::"n"(32 * kCtaGather) : "memory");
@@ -56,9 +67,10 @@ __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefe
 // last entry, +inf while the list is not full (the register-worklist kernel's rule).
 // LREG: worklist entries per lane of warp 0 (L <= 32 LREG).
 template <typename S, int DC, int SPL, int LREG, bool IQ>
-__global__ void __launch_bounds__(kCtaThreads, DC == 0 && LREG <= 4 ? 4 : 3) search_cta_kernel(SearchArgs a, bool strict) {
+__global__ void __launch_bounds__(kCtaThreads, LREG <= 4 ? 4 : 3) search_cta_kernel(SearchArgs a, bool strict) {
     extern __shared__ __align__(16) unsigned char smem[];
-    constexpr uint32_t    G     = Layout<S, DC>::kG;
+    constexpr int         M     = CtaRows<S, DC>::kM;
+    constexpr uint32_t    G     = M * Layout<S, DC>::kP;
     constexpr uint32_t    SLOTS = SPL * 32;
     constexpr uint32_t    kDone = 0xFFFFFFFFu;
     const float           kInf  = __int_as_float(0x7f800000);
@@ -264,7 +276,7 @@ __global__ void __launch_bounds__(kCtaThreads, DC == 0 && LREG <= 4 ? 4 : 3) sea
             if (ctrl) fetch_row(entry);
             if (warp == 1) {
                 const float d0 =
-                    dist_group<S, DC, IQ>(qv, a.store, a.scale, [&](int) { return entry; }, 1, a.D, lane);
+                    dist_group<S, DC, IQ, M>(qv, a.store, a.scale, [&](int) { return entry; }, 1, a.D, lane);
                 if (lane == 0) ctl[1] = __float_as_uint(d0);
             }
             __syncthreads();  // the entry's distance
@@ -319,10 +331,10 @@ __global__ void __launch_bounds__(kCtaThreads, DC == 0 && LREG <= 4 ? 4 : 3) sea
                 const uint32_t beg = min(cnt, (warp - 1u) * per), end = min(cnt, beg + per);
                 for (uint32_t g0 = beg; g0 < end; g0 += G) {
                     const int      gc = (int)min(G, end - g0);
-                    const float    y  = dist_group<S, DC, IQ>(
+                    const float    y  = dist_group<S, DC, IQ, M>(
                         qv, a.store, a.scale, [&](int j) { return nb_id[slot_of(g0 + (uint32_t)j)]; }, gc, a.D, lane);
-                    const uint32_t vi = round_row_of_lane<S, DC>(lane);
-                    if (round_writer<S, DC>(lane) && (int)vi < gc) nb_d[slot_of(g0 + vi)] = y;
+                    const uint32_t vi = round_row_of_lane<S, DC, M>(lane);
+                    if (round_writer<S, DC, M>(lane) && (int)vi < gc) nb_d[slot_of(g0 + vi)] = y;
                 }
                 __syncthreads();  // the distances are there, and the previous merge is done
                 if (ctrl) {
@@ -361,15 +373,16 @@ __global__ void __launch_bounds__(kCtaThreads, DC == 0 && LREG <= 4 ? 4 : 3) sea
         if (a.out_ids != nullptr) {
             if (a.rerank) {
                 // exact FP32 distances of the final worklist, sorted (dist, position)
-                constexpr uint32_t  GF = Layout<StoreF32, DC>::kG;
+                constexpr int       MF = 4;
+                constexpr uint32_t  GF = MF * Layout<StoreF32, DC>::kP;
                 Query<StoreF32, DC> qf;
                 load_query<StoreF32, DC>(qf, a.queries + (uint64_t)q * a.D, a.D, lane);
                 for (uint32_t g0 = warp * GF; g0 < n; g0 += GF * (kCtaThreads / 32u)) {
                     const int      gc = (int)min(GF, n - g0);
-                    const float    y  = dist_group<StoreF32, DC>(
+                    const float    y  = dist_group<StoreF32, DC, false, MF>(
                         qf, a.vecs_f32, nullptr, [&](int j) { return wl_id[g0 + j] & ~kVisitedBit; }, gc, a.D, lane);
-                    const uint32_t vi = round_row_of_lane<StoreF32, DC>(lane);
-                    if (round_writer<StoreF32, DC>(lane) && (int)vi < gc) keys[g0 + vi] = make_key(y, g0 + vi);
+                    const uint32_t vi = round_row_of_lane<StoreF32, DC, MF>(lane);
+                    if (round_writer<StoreF32, DC, MF>(lane) && (int)vi < gc) keys[g0 + vi] = make_key(y, g0 + vi);
                 }
                 __syncthreads();
                 for (uint32_t i = tid; i < n; i += kCtaThreads) {

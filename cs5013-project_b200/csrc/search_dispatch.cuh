@@ -1,8 +1,7 @@
 // search_dispatch.cuh -- picks the search kernel instantiation for a launch:
 // register worklist (search_reg.cuh) for L <= 64 at D <= 128 and R <= 64,
 // shared-memory worklist (search_impl.cuh) otherwise, a CTA per query (search_cta.cuh)
-// for small batches of either, and the launch-bound
-// variant chosen by the autotuner.
+// for small batches of either, and the launch-bound variant chosen by the autotuner.
 #pragma once
 #include "search_cta.cuh"
 #include "search_reg.cuh"
@@ -74,15 +73,15 @@ static cudaError_t launch_r(const SearchArgs& a, int variant, int sms, cudaStrea
 
 // Batches served by a CTA per query (search_cta.cuh): up to as many queries as keep it
 // ahead of a warp per query, which needs many to fill the chip but then does more of them.
-// Measured on 148 SMs, CTA / warp per query in us (10 to 1,500 queries):
-//   worklist in registers otherwise (L <= 64): uint8 1M x 128, L = 64: 1 query 92 / 114,
-//     300 queries 254 / 305, 590 320 / 373, 900 400 / 415, 1,500 509 / 422; uint8 L = 32: 590
-//     118 / 134, 700 148 / 135;
-//   L <= 128, or wider rows or lists: FP32 200k x 96, L = 100: 1 query 125 / 211, 590 300 /
-//     479, 1,000 371 / 481, 1,200 494 / 476; BF16 100k x 256, L = 128 with rerank: 1 query
-//     241 / 493, 1,000 976 / 1,074, 1,200 1,126 / 1,110;
-//   L <= 256 (more registers, fewer CTAs): FP32 L = 200: 1 query 194 / 319, 300 248 / 416, 590
-//     451 / 429.
+// Measured on 148 SMs, CTA / warp per query in us:
+//   worklist in registers otherwise (L <= 64): uint8 1M x 128, L = 64: 1 query 88 / 114, 300
+//     queries 247 / 305, 590 322 / 373; uint8 L = 32: 1 query 50 / 58, 590 114 / 134 (with 8
+//     rows a round instead of 4, 700 queries took 148 / 135);
+//   L <= 128, or wider rows or lists: FP32 200k x 96, L = 100: 1 query 116 / 211, 590 298 /
+//     479, 1,000 365 / 481 (1,200: 494 / 476); BF16 100k x 256, L = 128 with rerank: 1 query
+//     242 / 493, 590 563 / 981, 1,000 837 / 1,074 (1,200: 1,126 / 1,110);
+//   L <= 256 (more registers, fewer CTAs): FP32 L = 200: 1 query 189 / 319, 300 239 / 416 (590:
+//     451 / 429).
 inline bool small_batch(const SearchArgs& a, int sms) {
     if (a.beam == 2 || a.L > kCtaMaxL) return false;
     const uint64_t per_sm = a.L > 128 ? 3 : (a.L > 64 || a.D > 128 || a.R > 64 ? 7 : 4);
