@@ -236,15 +236,13 @@ struct vann_index {
     // per-query L / k arrays of the vann_search_uneven call in progress
     const uint32_t* pending_Lq = nullptr;
     const uint32_t* pending_kq = nullptr;
-    // launch-bound variant of the build and insert searches per row format (-1: not timed yet)
-    int build_variant[4] = {-1, -1, -1, -1};
     // autotuned search variant per (store, rerank, beam, L)
     std::map<std::tuple<uint32_t, uint32_t, uint32_t, uint32_t>, int> tuned;
 
     static uint32_t beam_of(const vann_search_params& sp) { return sp.beam == 2 ? 2u : 1u; }
     int variant_for(const vann_search_params& sp) const {
         auto it = tuned.find(std::make_tuple(sp.store, sp.rerank ? 1u : 0u, beam_of(sp), sp.L));
-        return it == tuned.end() ? 0 : it->second;
+        return it == tuned.end() ? -1 : it->second;
     }
 
     // search order of large batches (distance keys, then the order), one workspace per
@@ -519,33 +517,7 @@ struct vann_index {
             sstore        = VANN_STORE_U8;
             a.int_queries = 1;  // the batch's rows are rows of the exact copy
         }
-        // the first large batch of each row format times the launch-bound variants
-        // (the same search each time: the expansion lists do not depend on the variant)
-        if (build_variant[sstore] < 0 && count >= 4096) {
-            cudaEvent_t e0, e1;
-            VCHECK(cudaEventCreate(&e0));
-            VCHECK(cudaEventCreate(&e1));
-            float best_ms = 1e30f;
-            int   best    = 0;
-            for (int v = 0; v < vann::search_variants(); ++v) {
-                a.counter = next_counter(st);
-                VCHECK(cudaEventRecord(e0, st));
-                VCHECK(vann::launch_search(a, sstore, num_sms, st, v));
-                VCHECK(cudaEventRecord(e1, st));
-                VCHECK(cudaEventSynchronize(e1));
-                float ms = 0.f;
-                VCHECK(cudaEventElapsedTime(&ms, e0, e1));
-                if (ms < best_ms) {
-                    best_ms = ms;
-                    best    = v;
-                }
-            }
-            cudaEventDestroy(e0);
-            cudaEventDestroy(e1);
-            build_variant[sstore] = best;
-            a.counter = next_counter(st);
-        }
-        VCHECK(vann::launch_search(a, sstore, num_sms, st, std::max(build_variant[sstore], 0)));
+        VCHECK(vann::launch_search(a, sstore, num_sms, st));
 
         vann::PruneArgs pa{};
         pa.vecs = vecs;

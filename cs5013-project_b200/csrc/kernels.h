@@ -49,7 +49,8 @@ struct SearchArgs {
     uint32_t*       status;
 };
 
-cudaError_t launch_search(const SearchArgs& a, int store, int num_sms, cudaStream_t st, int variant = 0);
+// variant: a compiled launch variant, or -1 for the one chosen by format and batch size
+cudaError_t launch_search(const SearchArgs& a, int store, int num_sms, cudaStream_t st, int variant = -1);
 int         search_variants();
 
 // RobustPrune over candidates A (expansion list or reverse entries) merged with

@@ -88,6 +88,31 @@ inline bool small_batch(const SearchArgs& a, int sms) {
     return a.nq <= per_sm * (uint64_t)sms;
 }
 
+// Launch-bound variant of a search that was not autotuned: the register cap trades
+// resident warps for spills, so it depends on the row format's registers and on how many
+// warps the batch can fill.  Measured (10,000 / 3,000 queries, ms at a cap for 6 blocks per SM
+// against the choice):
+//   FP8 (its conversions need the registers): 5 blocks.  L = 40..64: 1.27 -> 1.13 / 0.64 ->
+//     0.53, L = 100: 2.29 -> 1.88;
+//   register worklist, up to 24 queries per SM (every query resident): 5.  uint8 L = 64 on
+//     1M x 128: 0.458 -> 0.439, BF16 L = 32: 0.386 -> 0.373;
+//   register worklist, more than 36: uint8 8 (L = 32: 0.472 -> 0.458, L = 64 on 1M x 96: 0.750
+//     -> 0.716), FP32 7 (L = 32: 0.831 -> 0.800), BF16 8 for L <= 32 (0.687 -> 0.657);
+//   shared-memory worklist, uint8 and FP32: 7 (uint8 L = 100: 1.217 -> 1.173, FP32 L = 199 on
+//     10k rows: 1.562 -> 1.538; 8 spills: 1.406, 1.832).
+template <typename S>
+static int default_variant(const SearchArgs& a, int sms) {
+    constexpr int k5 = 2, k6 = 0, k7 = 3, k8 = 4;
+    if (S::kScaled) return k5;
+    if (S::kPQ) return k6;
+    constexpr bool f32 = !S::kInt && S::kElems == 4;
+    if (a.L > 64 || a.R > 64) return (S::kInt || f32) && a.nq > 24ull * (uint64_t)sms ? k7 : k6;
+    if (a.nq <= 24ull * (uint64_t)sms) return k5;
+    if (a.nq <= 36ull * (uint64_t)sms) return k6;
+    if (S::kInt) return k8;
+    return f32 ? k7 : (a.L <= 32 ? k8 : k6);
+}
+
 template <typename S>
 static cudaError_t launch_store(const SearchArgs& a, int variant, int sms, cudaStream_t st) {
     if (a.D % S::kElems != 0) return cudaErrorInvalidValue;
@@ -100,6 +125,7 @@ static cudaError_t launch_store(const SearchArgs& a, int variant, int sms, cudaS
             return launch_cta<S, 2>(a, sms, st);
         }
     }
+    if (variant < 0) variant = default_variant<S>(a, sms);
     if (a.D <= 128) return launch_r<S, 0>(a, variant, sms, st);
     if (a.D <= 256) return launch_r<S, 1>(a, variant, sms, st);
     return launch_r<S, 2>(a, variant, sms, st);
