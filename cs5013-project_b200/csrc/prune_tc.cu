@@ -7,7 +7,8 @@
 // sums in any order, and the integer identity |x|^2 + |y|^2 - 2 x.y, give the
 // same value: the decisions are bit-identical to the FP32 path.
 //
-// One CTA of 4 warps (the 128 TMEM lanes) prunes one node at a time:
+// One CTA (4 warps for the 128 TMEM lanes, 8 in the larger classes) prunes one node at a
+// time:
 //   1. candidate ids (A then B, as in prune.cu) with their distances to the node
 //      (given by the search, or computed exactly from the uint8 rows);
 //   2. stable order by (distance, candidate index): a candidate's rank is the count of
@@ -51,7 +52,10 @@
 namespace vann {
 namespace {
 
-constexpr uint32_t kThreads  = 128;  // 4 warps = the 128 TMEM lanes
+// Threads of a CTA: 4 warps (the 128 TMEM lanes) for the smallest class, whose nodes in
+// flight fill the SM; 8 for the larger ones, where few CTAs fit and each phase's length
+// counts (two warps share a quarter of the lanes and split the columns).
+__host__ __device__ constexpr uint32_t tc_threads(uint32_t maxc) { return maxc == 128u ? 128u : 256u; }
 constexpr uint32_t kMaxR     = 128;
 constexpr long long kSpinCycles = 2000000000ll;  // ~1 s bound on an MMA completion wait
 
@@ -159,7 +163,7 @@ struct TcLayout {
         l.nrm    = l.sd + 4 * maxc;
         l.pby    = l.nrm + (f16 ? 0u : 4 * maxc);  // [maxc / 32][maxc] bits of the candidates that prune t
         l.bmask  = l.pby + maxc * maxc / 8;        // sorted positions holding B candidates
-        l.chosen = l.bmask + 16 * ((maxc + kThreads - 1) / kThreads);  // the node's new list
+        l.chosen = l.bmask + 4 * ((maxc + 255u) / 256u * 8u);  // the node's new list
         l.pairs  = l.chosen + 4 * kMaxR;                               // undecided pairs (f16 rows)
         l.bar    = l.pairs + (f16 ? 4 * kPairs(maxc) : 0u);
         l.misc   = l.bar + 8;
@@ -198,11 +202,13 @@ __device__ __forceinline__ float half_warp_dist(const float* x, const float* y, 
 // null); nodes with more than MAXC candidates go to out_list.  COLS: TMEM columns per
 // CTA, the width of a Gram tile.  F16: float rows (the filter described above).
 template <uint32_t MAXC, uint32_t COLS, bool F16>
-__global__ void __launch_bounds__(kThreads, MAXC == 128 ? 8 : 1)
+__global__ void __launch_bounds__(tc_threads(MAXC), MAXC == 128 ? 8 : (MAXC == 256 ? (F16 ? 2 : 4) : 1))
     prune_tc_kernel(PruneArgs a, uint32_t* counter, const uint32_t* in_list, const uint32_t* in_count,
                     uint32_t* out_list, uint32_t* out_count) {
-    constexpr uint32_t KPT = (MAXC + kThreads - 1) / kThreads;  // candidates per thread
-    constexpr uint32_t kB  = 0x80000000u;      // sid: a B candidate (ids are below 2^31)
+    constexpr uint32_t kThreads = tc_threads(MAXC);
+    constexpr uint32_t kSplit   = kThreads / 128;                    // warps per quarter of the TMEM lanes
+    constexpr uint32_t KPT      = (MAXC + kThreads - 1) / kThreads;  // candidates per thread
+    constexpr uint32_t kB       = 0x80000000u;                       // sid: a B candidate (ids are below 2^31)
     extern __shared__ __align__(1024) unsigned char smem[];
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     const uint64_t nwork = in_list ? (uint64_t)*reinterpret_cast<volatile const uint32_t*>(in_count) : a.n_nodes;
@@ -373,11 +379,11 @@ __global__ void __launch_bounds__(kThreads, MAXC == 128 ? 8 : 1)
                 r[q]             = __popc(__match_any_sync(0xffffffffu, b[q]) & ((1u << lane) - 1u));
             }
             const uint32_t used = (nc + kThreads - 1) / kThreads;  // candidates in use per thread
-            for (uint32_t c0 = 0; c0 < nc; c0 += 32) {             // the warp's own chunk: 128 q + 32 warp
+            for (uint32_t c0 = 0; c0 < nc; c0 += 32) {  // the warp's own chunk: kThreads q + 32 warp
                 const uint4* dj = reinterpret_cast<const uint4*>(cd + c0);
                 uint32_t     thr[KPT];
 #pragma unroll
-                for (uint32_t q = 0; q < KPT; ++q) thr[q] = b[q] + (c0 < 128u * q + 32u * warp ? 1u : 0u);
+                for (uint32_t q = 0; q < KPT; ++q) thr[q] = b[q] + (c0 < kThreads * q + 32u * warp ? 1u : 0u);
 #pragma unroll
                 for (uint32_t j = 0; j < 8; ++j) {
                     const uint4 x = dj[j];
@@ -442,9 +448,9 @@ __global__ void __launch_bounds__(kThreads, MAXC == 128 ? 8 : 1)
         if (a.consistent) {
 #pragma unroll
             for (uint32_t q = 0; q < KPT; ++q) {
-                const uint32_t t    = 128u * q + tid;
+                const uint32_t t    = kThreads * q + tid;
                 const uint32_t bits = __ballot_sync(0xffffffffu, t < m && (sid[t] & kB) != 0u);
-                if (lane == 0) bmask[4u * q + warp] = bits;
+                if (lane == 0) bmask[(kThreads / 32u) * q + warp] = bits;
             }
         }
         cp_async_wait_all();
@@ -483,7 +489,7 @@ __global__ void __launch_bounds__(kThreads, MAXC == 128 ? 8 : 1)
         // --- 5. bits of the candidates that prune t
         bool late = false;
         for (uint32_t r = 0; r < nb; ++r) {
-            const uint32_t t = 128u * r + tid;
+            const uint32_t t = 128u * r + (tid & 127u);
             // "u prunes t" is alpha * d(u, t) <= d(node, t) in FP32, with d(u, t) the exact
             // integer Y = |u|^2 + |t|^2 - 2 u.t (< 2^24, so FP32 holds it exactly).  fl(Y *
             // alpha) does not decrease as Y grows, so the test is Y <= Ymax(t), the largest
@@ -513,7 +519,7 @@ __global__ void __launch_bounds__(kThreads, MAXC == 128 ? 8 : 1)
                 }
                 if (a.consistent && (sid[t] & kB)) keep = 0u;
             }
-            const uint32_t last  = 128u * r + 32u * warp + 31u;  // the warp's last candidate
+            const uint32_t last  = 128u * r + 32u * (warp & 3u) + 31u;  // the warp's last candidate
             const uint32_t ncols = min(m, 128u * (r + 1u));
             for (uint32_t c = 0; COLS * c < ncols; ++c) {
                 if (r != 0 || c != 0) {
@@ -528,7 +534,7 @@ __global__ void __launch_bounds__(kThreads, MAXC == 128 ? 8 : 1)
                 phase ^= 1u;
                 tc_fence_after();
 #pragma unroll 1
-                for (uint32_t c32 = 0; c32 < COLS; c32 += 32u) {
+                for (uint32_t c32 = 32u * (warp >> 2); c32 < COLS; c32 += 32u * kSplit) {
                     const uint32_t u0 = COLS * c + c32;
                     if (u0 >= m || u0 > last) break;
                     uint32_t word = 0, open = 0;  // open: undecided (float rows)
@@ -536,7 +542,7 @@ __global__ void __launch_bounds__(kThreads, MAXC == 128 ? 8 : 1)
                     for (uint32_t h = 0; h < 32u; h += 16u) {
                         if (u0 + h < m) {
                             uint32_t g[16];
-                            tmem_ld16(tmem + ((32u * warp) << 16) + c32 + h, g);
+                            tmem_ld16(tmem + ((32u * (warp & 3u)) << 16) + c32 + h, g);
 #pragma unroll
                             for (uint32_t k = 0; k < 16; k += 4) {
                                 if constexpr (F16) {
@@ -686,7 +692,7 @@ cudaError_t launch_tc(const PruneArgs& a, uint32_t* counter, const uint32_t* in_
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
     uint64_t grid = (uint64_t)per_sm * num_sms;
     if (grid > max_nodes) grid = max_nodes;
-    kern<<<(unsigned)grid, kThreads, smem, st>>>(a, counter, in_list, in_count, out_list, out_count);
+    kern<<<(unsigned)grid, tc_threads(MAXC), smem, st>>>(a, counter, in_list, in_count, out_list, out_count);
     return cudaGetLastError();
 }
 
