@@ -124,7 +124,6 @@ struct StagedArgs {
     uint32_t*       out_ids;    // nq x L: graph id, or 0x80000000 | insert-list row
     float*          out_d;      // nq x L
     float*          out_vecs;   // nq x L x D or null
-    uint32_t        p2;         // set by the launcher
 };
 cudaError_t launch_staged_merge(const StagedArgs& a, int num_sms, cudaStream_t st);
 
