@@ -283,9 +283,10 @@ struct vann_index {
             b->release();
     }
 
-    uint32_t* next_counter(cudaStream_t st, bool zero = true) {
+    // a slot of the counter ring, its first `zeroed` of 32 words cleared on the stream
+    uint32_t* next_counter(cudaStream_t st, uint32_t zeroed = 1) {
         uint32_t* c = counters + (ring_pos++ % kCounterRing) * 32;
-        if (zero) VCHECK(cudaMemsetAsync(c, 0, sizeof(uint32_t), st));
+        if (zeroed) VCHECK(cudaMemsetAsync(c, 0, sizeof(uint32_t) * zeroed, st));
         return c;
     }
 
@@ -420,37 +421,32 @@ struct vann_index {
             pa.vecs_u8 = static_cast<const uint8_t*>(store[3]);
             pa.gate    = u8_inexact();
         }
-        // lists: [0, n] rev hand-off + count, [n+1, 2n+2) final hand-off + count, then the passes' scratch
-        ovf.ensure(sizeof(uint32_t) * (4 * n + 8));
-        uint32_t*       rev_list   = ovf.as<uint32_t>();
-        uint32_t*       rev_count  = rev_list + n;
-        uint32_t*       last_list  = rev_list + n + 1;
-        uint32_t*       last_count = last_list + n;
-        uint32_t*       ws         = last_count + 1;
-        const uint32_t* in_list    = nullptr;  // every node
+        // hand-off lists: from the reverse kernel, from the last tensor-core pass, and two
+        // between the passes.  Every counter and count of the call is in one zeroed slot
+        // (a memset each was 13 of the 36 device operations of an insert of ten rows).
+        ovf.ensure(sizeof(uint32_t) * 4 * n);
+        uint32_t*       rev_list  = ovf.as<uint32_t>();
+        uint32_t*       last_list = rev_list + n;
+        uint32_t*       ws        = last_list + n;
+        uint32_t*       c         = next_counter(st, 16);  // [0..3] passes, [4] rev, [5] prune_kernel
+        uint32_t*       rev_count = c + 6;
+        uint32_t*       last_count = c + 7;
+        uint32_t*       counts     = c + 8;                // [8..10] between the passes
+        const uint32_t* in_list    = nullptr;              // every node
         const uint32_t* in_count   = nullptr;
         if (rev) {
-            VCHECK(cudaMemsetAsync(rev_count, 0, sizeof(uint32_t), st));
+            pa.counter = c + 4;
             VCHECK(vann::launch_prune_rev(pa, u8_exact(st), rev_list, rev_count, num_sms, st));
-            pa.counter = next_counter(st);
-            in_list    = rev_list;
-            in_count   = rev_count;
+            in_list  = rev_list;
+            in_count = rev_count;
         }
-        if (tc) {
-            uint32_t* tc_counters = next_counter(st);  // one per pass
-            VCHECK(cudaMemsetAsync(tc_counters + 1, 0, 3 * sizeof(uint32_t), st));
-            VCHECK(vann::launch_prune_tc(pa, in_list, in_count, last_list, last_count, ws, tc_counters, num_sms,
-                                         st));
-            in_list  = last_list;
-            in_count = last_count;
-        } else if (f16) {
-            uint32_t* f16_counters = next_counter(st);  // one per pass
-            VCHECK(cudaMemsetAsync(f16_counters + 1, 0, 2 * sizeof(uint32_t), st));
-            VCHECK(vann::launch_prune_f16(pa, in_list, in_count, last_list, last_count, ws, f16_counters, num_sms,
-                                          st));
+        if (tc || f16) {
+            VCHECK((tc ? vann::launch_prune_tc : vann::launch_prune_f16)(pa, in_list, in_count, last_list, last_count,
+                                                                         ws, c, counts, num_sms, st));
             in_list  = last_list;
             in_count = last_count;
         }
+        pa.counter  = c + 5;
         pa.in_list  = in_list;
         pa.in_count = in_count;
         VCHECK(vann::launch_prune(pa, num_sms, st));
@@ -536,7 +532,6 @@ struct vann_index {
         pa.a_stride = MV;
         pa.use_b = 1;
         pa.consistent = 0;
-        pa.counter = next_counter(st);
         pa.status = status;
         run_prune(pa, st);
 
@@ -624,7 +619,6 @@ struct vann_index {
             ra.skip_empty = 0;
             ra.consistent = 0;
         }
-        ra.counter = next_counter(st);
         run_prune(ra, st);
         consistent = true;
     }
@@ -1099,7 +1093,7 @@ vann_status vann_search_stats(vann_index* h, const float* d_queries, uint64_t nq
             }
         }
         // the order kernel zeroes the counter, else a memset does
-        a.counter  = h->next_counter(S(stream), false);
+        a.counter  = h->next_counter(S(stream), 0);
         bool chain = false;
         a.order    = h->search_order(d_queries, nq, S(stream), a.counter, &chain);
         if (a.order == nullptr) VCHECK(cudaMemsetAsync(a.counter, 0, sizeof(uint32_t), S(stream)));
@@ -1421,7 +1415,6 @@ vann_status vann_consolidate(vann_index* h, void* stream) {
             pa.a_stride = cap;
             pa.use_b = 0;
             pa.consistent = 0;
-            pa.counter = h->next_counter(st);
             pa.status = h->status;
             h->run_prune(pa, st);
         }

@@ -82,7 +82,7 @@ struct PruneArgs {
     int             use_b;       // include the node's current out-neighbours
     int             skip_empty;  // re-prune: skip nodes without reverse entries
     int             consistent;  // B lists are alpha-consistent: skip B-B checks
-    uint32_t*       counter;     // work counter, zeroed before launch
+    uint32_t*       counter;     // work counter, zeroed before launch (set by the caller of the launches)
     uint32_t*       status;
     // tensor-core passes (prune_tc.cu) and the hand-off between kernels
     const uint8_t*  vecs_u8;     // exact uint8 rows (or null)
@@ -95,17 +95,18 @@ struct PruneArgs {
 // prune_kernel: every node, or the listed slots when a.in_count is set.
 cudaError_t launch_prune(const PruneArgs& a, int num_sms, cudaStream_t st);
 bool        prune_tc_supported(uint32_t D, uint32_t R);
-// Tensor-core passes over in_list (every node when null); leftovers to out_list.
-// ws: 2 * n_nodes + 4 words of scratch; counters: four zeroed work counters.
+// Tensor-core passes over in_list (every node when null); leftovers to out_list.  ws:
+// 2 * n_nodes words of scratch; counters, counts and out_count zeroed: four work counters
+// and three counts of nodes handed on.
 cudaError_t launch_prune_tc(const PruneArgs& a, const uint32_t* in_list, const uint32_t* in_count,
-                            uint32_t* out_list, uint32_t* out_count, uint32_t* ws, uint32_t* counters, int num_sms,
-                            cudaStream_t st);
+                            uint32_t* out_list, uint32_t* out_count, uint32_t* ws, uint32_t* counters,
+                            uint32_t* counts, int num_sms, cudaStream_t st);
 // The same passes over float rows (D <= 128): a Gram matrix of f16 rows as a filter, pairs
-// it cannot decide by their FP32 distances.  ws as above; counters: three zeroed ones.
+// it cannot decide by their FP32 distances.
 bool        prune_f16_supported(uint32_t D, uint32_t R);
 cudaError_t launch_prune_f16(const PruneArgs& a, const uint32_t* in_list, const uint32_t* in_count,
-                             uint32_t* out_list, uint32_t* out_count, uint32_t* ws, uint32_t* counters, int num_sms,
-                             cudaStream_t st);
+                             uint32_t* out_list, uint32_t* out_count, uint32_t* ws, uint32_t* counters,
+                             uint32_t* counts, int num_sms, cudaStream_t st);
 // Reverse re-prune of consistent lists, one warp per node (prune_rev.cu): nodes
 // with more than 128 candidates or 8 reverse sources are handed on in out_list.
 // u8: distances from a.vecs_u8 (the host has read that every row is exact).

@@ -702,11 +702,12 @@ cudaError_t launch_tc(const PruneArgs& a, uint32_t* counter, const uint32_t* in_
 // SM, when its shared memory fits: D <= 160), each over the nodes the previous one
 // handed on.  The first pass takes in_list[0 .. *in_count) (every node when null);
 // what the last cannot take goes to out_list for prune_kernel.  A launch of no more
-// nodes than SMs has nothing to fill with small passes: it goes straight to the last.
-// ws: 2 * n_nodes + 4 words of device scratch; counters: four zeroed work counters.
+// nodes than SMs has nothing to fill with small passes and goes straight to the last; one
+// of no more than the 256 class holds at once (4 per SM) takes that and the last.
+// ws: 2 * n_nodes words of device scratch; counters, counts, out_count: zeroed.
 cudaError_t launch_prune_tc(const PruneArgs& a, const uint32_t* in_list, const uint32_t* in_count,
-                            uint32_t* out_list, uint32_t* out_count, uint32_t* ws, uint32_t* counters, int num_sms,
-                            cudaStream_t st) {
+                            uint32_t* out_list, uint32_t* out_count, uint32_t* ws, uint32_t* counters,
+                            uint32_t* counts, int num_sms, cudaStream_t st) {
     if (a.n_nodes == 0) return cudaSuccess;
     if (!prune_tc_supported(a.D, a.R) || !a.vecs_u8 || !a.gate || !out_list || !out_count)
         return cudaErrorInvalidValue;
@@ -715,42 +716,48 @@ cudaError_t launch_prune_tc(const PruneArgs& a, const uint32_t* in_list, const u
     if (e != cudaSuccess) return e;
     e = cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     if (e != cudaSuccess) return e;
-    const bool last768 = TcLayout::make(a.D, 768, false).bytes <= (uint32_t)max_optin;
-    if ((e = cudaMemsetAsync(out_count, 0, sizeof(uint32_t), st)) != cudaSuccess) return e;
-    if (last768 && a.n_nodes <= (uint64_t)num_sms)
-        return launch_tc<768, 128>(a, counters, in_list, in_count, out_list, out_count, a.n_nodes, num_sms, st);
-    // the hand-off lists alternate between two halves of ws; their counts sit together
-    uint32_t* list[2] = {ws, ws + a.n_nodes};
-    uint32_t* cnt     = ws + 2 * a.n_nodes;  // one per hand-off
-    if ((e = cudaMemsetAsync(cnt, 0, 3 * sizeof(uint32_t), st)) != cudaSuccess) return e;
-    e = launch_tc<128, 64>(a, counters, in_list, in_count, list[0], cnt, a.n_nodes, num_sms, st);
+    const uint64_t n       = a.n_nodes;
+    const bool     last768 = TcLayout::make(a.D, 768, false).bytes <= (uint32_t)max_optin;
+    uint32_t*      list[2] = {ws, ws + n};
+    if (last768 && n <= (uint64_t)num_sms)
+        return launch_tc<768, 128>(a, counters, in_list, in_count, out_list, out_count, n, num_sms, st);
+    if (last768 && n <= 4ull * (uint64_t)num_sms) {
+        e = launch_tc<256, 128>(a, counters, in_list, in_count, list[0], counts, n, num_sms, st);
+        if (e != cudaSuccess) return e;
+        return launch_tc<768, 128>(a, counters + 1, list[0], counts, out_list, out_count, n, num_sms, st);
+    }
+    e = launch_tc<128, 64>(a, counters, in_list, in_count, list[0], counts, n, num_sms, st);
     if (e != cudaSuccess) return e;
-    e = launch_tc<256, 128>(a, counters + 1, list[0], cnt, list[1], cnt + 1, a.n_nodes, num_sms, st);
+    e = launch_tc<256, 128>(a, counters + 1, list[0], counts, list[1], counts + 1, n, num_sms, st);
     if (e != cudaSuccess) return e;
-    if (!last768) return launch_tc<512, 128>(a, counters + 2, list[1], cnt + 1, out_list, out_count, a.n_nodes, num_sms, st);
-    e = launch_tc<512, 128>(a, counters + 2, list[1], cnt + 1, list[0], cnt + 2, a.n_nodes, num_sms, st);
+    if (!last768)
+        return launch_tc<512, 128>(a, counters + 2, list[1], counts + 1, out_list, out_count, n, num_sms, st);
+    e = launch_tc<512, 128>(a, counters + 2, list[1], counts + 1, list[0], counts + 2, n, num_sms, st);
     if (e != cudaSuccess) return e;
-    return launch_tc<768, 128>(a, counters + 3, list[0], cnt + 2, out_list, out_count, a.n_nodes, num_sms, st);
+    return launch_tc<768, 128>(a, counters + 3, list[0], counts + 2, out_list, out_count, n, num_sms, st);
 }
 
-// The same over float rows: passes of 128, 256 and 576 candidates.  ws: 2 * n_nodes + 2
-// words of device scratch; counters: three zeroed work counters.
+// The same over float rows: passes of 128, 256 and 576 candidates.
 cudaError_t launch_prune_f16(const PruneArgs& a, const uint32_t* in_list, const uint32_t* in_count,
-                             uint32_t* out_list, uint32_t* out_count, uint32_t* ws, uint32_t* counters, int num_sms,
-                             cudaStream_t st) {
+                             uint32_t* out_list, uint32_t* out_count, uint32_t* ws, uint32_t* counters,
+                             uint32_t* counts, int num_sms, cudaStream_t st) {
     if (a.n_nodes == 0) return cudaSuccess;
     if (!prune_f16_supported(a.D, a.R) || !out_list || !out_count) return cudaErrorInvalidValue;
-    cudaError_t e = cudaMemsetAsync(out_count, 0, sizeof(uint32_t), st);
+    const uint64_t n       = a.n_nodes;
+    uint32_t*      list[2] = {ws, ws + n};
+    if (n <= (uint64_t)num_sms)
+        return launch_tc<576, 128, true>(a, counters, in_list, in_count, out_list, out_count, n, num_sms, st);
+    cudaError_t     e   = cudaSuccess;
+    const uint32_t *il = in_list, *ic = in_count;
+    if (n > 4ull * (uint64_t)num_sms) {
+        e  = launch_tc<128, 64, true>(a, counters, il, ic, list[0], counts, n, num_sms, st);
+        il = list[0];
+        ic = counts;
+        if (e != cudaSuccess) return e;
+    }
+    e = launch_tc<256, 128, true>(a, counters + 1, il, ic, list[1], counts + 1, n, num_sms, st);
     if (e != cudaSuccess) return e;
-    if (a.n_nodes <= (uint64_t)num_sms)
-        return launch_tc<576, 128, true>(a, counters, in_list, in_count, out_list, out_count, a.n_nodes, num_sms, st);
-    uint32_t *list1 = ws, *list2 = ws + a.n_nodes, *cnt = ws + 2 * a.n_nodes;
-    if ((e = cudaMemsetAsync(cnt, 0, 2 * sizeof(uint32_t), st)) != cudaSuccess) return e;
-    e = launch_tc<128, 64, true>(a, counters, in_list, in_count, list1, cnt, a.n_nodes, num_sms, st);
-    if (e != cudaSuccess) return e;
-    e = launch_tc<256, 128, true>(a, counters + 1, list1, cnt, list2, cnt + 1, a.n_nodes, num_sms, st);
-    if (e != cudaSuccess) return e;
-    return launch_tc<576, 128, true>(a, counters + 2, list2, cnt + 1, out_list, out_count, a.n_nodes, num_sms, st);
+    return launch_tc<576, 128, true>(a, counters + 2, list[1], counts + 1, out_list, out_count, n, num_sms, st);
 }
 
 }  // namespace vann
