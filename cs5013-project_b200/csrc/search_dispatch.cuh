@@ -88,29 +88,37 @@ inline bool small_batch(const SearchArgs& a, int sms) {
     return a.nq <= per_sm * (uint64_t)sms;
 }
 
-// Launch-bound variant of a search that was not autotuned: the register cap trades
-// resident warps for spills, so it depends on the row format's registers and on how many
-// warps the batch can fill.  Measured (10,000 / 3,000 queries, ms at a cap for 6 blocks per SM
-// against the choice):
-//   FP8 (its conversions need the registers): 5 blocks.  L = 40..64: 1.27 -> 1.13 / 0.64 ->
-//     0.53, L = 100: 2.29 -> 1.88;
-//   register worklist, up to 24 queries per SM (every query resident): 5.  uint8 L = 64 on
-//     1M x 128: 0.458 -> 0.439, BF16 L = 32: 0.386 -> 0.373;
-//   register worklist, more than 36: uint8 8 (L = 32: 0.472 -> 0.458, L = 64 on 1M x 96: 0.750
-//     -> 0.716), FP32 7 (L = 32: 0.831 -> 0.800), BF16 8 for L <= 32 (0.687 -> 0.657);
-//   shared-memory worklist, uint8 and FP32: 7 (uint8 L = 100: 1.217 -> 1.173, FP32 L = 199 on
-//     10k rows: 1.562 -> 1.538; 8 spills: 1.406, 1.832).
+// Launch-bound variant (blocks of 4 warps per SM) of a search that was not autotuned.  A
+// register cap trades resident warps for spills, so the choice depends on the row
+// format's registers and on how many warps the batch can fill: while every query fits
+// at once more registers cost nothing.  Measured, ms at 6 blocks against the choice:
+//   every query resident at 4 blocks (16 queries per SM): 4.  1,800 queries: uint8 L = 58
+//     0.176 / 0.167, FP8 L = 58 0.356 / 0.297, FP32 L = 120 0.677 / 0.647, BF16 0.678 / 0.632;
+//   FP8 otherwise (its conversions need the registers): 4 for R <= 32, else 5.  10k on 1M x
+//     128: L = 64 1.267 / 1.130, L = 100 2.290 / 1.884;
+//   up to 24 per SM: 5, 6 for R <= 32 (BF16 5).  3,000 on 1M x 128: uint8 L = 64 0.458 / 0.439,
+//     BF16 L = 32 0.386 / 0.373; 3,400, R = 48: uint8 L = 120 0.703 / 0.636;
+//   up to 36: register worklist 6 (uint8 with R > 32: 5, 0.341 / 0.318), else as below;
+//   more, register worklist: uint8 8 (10k on 1M: L = 32 0.472 / 0.458, 1M x 96 L = 64 0.750 /
+//     0.716), FP32 7 for R > 32 (0.831 / 0.800; 10k rows 0.375 / 0.388), BF16 7 for L <= 32 or
+//     R <= 32 (0.687 / 0.676, 0.872 / 0.844);
+//   more, shared-memory worklist: uint8 and FP32 7 (uint8 L = 100 1.217 / 1.173, FP32 L = 199 on
+//     10k rows 1.562 / 1.538; 8 spills: 1.406, 1.832), BF16 6.
 template <typename S>
 static int default_variant(const SearchArgs& a, int sms) {
-    constexpr int k5 = 2, k6 = 0, k7 = 3, k8 = 4;
-    if (S::kScaled) return k5;
+    constexpr int  k4 = 1, k5 = 2, k6 = 0, k7 = 3, k8 = 4;
+    constexpr bool f32 = !S::kInt && S::kElems == 4, bf16 = S::kElems == 8;
+    const uint64_t n = a.nq, m = (uint64_t)sms;
+    const bool     reg = a.L <= 64 && a.R <= 64, short_list = a.R <= 32;
     if (S::kPQ) return k6;
-    constexpr bool f32 = !S::kInt && S::kElems == 4;
-    if (a.L > 64 || a.R > 64) return (S::kInt || f32) && a.nq > 24ull * (uint64_t)sms ? k7 : k6;
-    if (a.nq <= 24ull * (uint64_t)sms) return k5;
-    if (a.nq <= 36ull * (uint64_t)sms) return k6;
+    if (n <= 16 * m) return k4;
+    if (S::kScaled) return short_list ? k4 : k5;
+    if (n <= 24 * m) return short_list && !(bf16 && reg) ? k6 : k5;
+    if (!reg) return S::kInt || f32 ? k7 : k6;
+    if (n <= 36 * m) return S::kInt && !short_list ? k5 : k6;
     if (S::kInt) return k8;
-    return f32 ? k7 : (a.L <= 32 ? k8 : k6);
+    if (f32) return short_list ? k6 : k7;
+    return a.L <= 32 || short_list ? k7 : k6;
 }
 
 template <typename S>
