@@ -99,8 +99,9 @@ typedef struct {
     uint32_t dim, degree;
     uint32_t consistent;   /* 1 when every adjacency list came from RobustPrune with alpha */
     uint64_t device_bytes; /* device memory held by the index */
-    uint64_t pruned_tc;    /* RobustPrune runs done with the Gram matrix on the tensor cores */
-    uint64_t pruned_cuda;  /* RobustPrune runs done on the CUDA cores (float rows, overflow) */
+    uint64_t pruned_tc;    /* RobustPrune runs decided by the exact integer Gram matrix on the tensor cores */
+    uint64_t pruned_cuda;  /* RobustPrune runs decided in FP32 or by the reverse kernel: float rows (the
+                              tensor cores only sort out the clear pairs), few-source re-prunes, overflow */
     uint64_t staged;       /* rows in the insert list (vann_stage_insert), not yet in the graph */
 } vann_info;
 
