@@ -295,8 +295,10 @@ __global__ void __launch_bounds__(kCtaThreads, LREG <= 4 ? 4 : 3) search_cta_ker
                         ++hops;
                         dg = dg < R ? dg : R;
                         adjw += dg;
-                        const bool seen = (bloom[h1 >> 5] >> (h1 & 31u)) & (bloom[h2 >> 5] >> (h2 & 31u)) & 1u;
-                        pass            = slot < dg && !seen && nid != skip;
+                        pass = slot < dg && nid != skip;
+                        // slots past the degree hold whatever was in memory: their filter
+                        // slots may lie outside the filter
+                        if (pass) pass = !((bloom[h1 >> 5] >> (h1 & 31u)) & (bloom[h2 >> 5] >> (h2 & 31u)) & 1u);
                         if (a.tomb != nullptr && pass) pass = !((__ldg(a.tomb + (nid >> 5)) >> (nid & 31u)) & 1u);
                         const uint32_t m = __ballot_sync(0xffffffffu, pass);
                         if (pass) nb_id[32u * sg + __popc(m & ((1u << lane) - 1u))] = nid;
