@@ -41,22 +41,26 @@ struct SmemLayout {
     }
 };
 
-__device__ __forceinline__ uint32_t upper_bound_f(const float* a, uint32_t n, float x) {
+// Distances are ordered by their bits throughout: they are non-negative, so that is their
+// order as numbers, and a row with a NaN in it sorts behind every other, +inf included (by
+// float comparisons a NaN is neither above nor below, so that the merge gave two entries
+// one place and left another unwritten).
+__device__ __forceinline__ uint32_t upper_bound_f(const float* a, uint32_t n, uint32_t x) {
     uint32_t lo = 0, hi = n;
     while (lo < hi) {
         uint32_t mid = (lo + hi) >> 1;
-        if (a[mid] <= x)
+        if (__float_as_uint(a[mid]) <= x)
             lo = mid + 1;
         else
             hi = mid;
     }
     return lo;
 }
-__device__ __forceinline__ uint32_t lower_bound_f(const float* a, uint32_t n, float x) {
+__device__ __forceinline__ uint32_t lower_bound_f(const float* a, uint32_t n, uint32_t x) {
     uint32_t lo = 0, hi = n;
     while (lo < hi) {
         uint32_t mid = (lo + hi) >> 1;
-        if (a[mid] < x)
+        if (__float_as_uint(a[mid]) < x)
             lo = mid + 1;
         else
             hi = mid;
@@ -193,9 +197,9 @@ __global__ void __launch_bounds__(128, MINB) search_kernel(SearchArgs a) {
 
             // candidates that cannot enter a full worklist are dropped before the
             // sort: with n == L a new entry with d >= wl_d[L-1] lands at >= L
-            const float tail = n == L ? wl_d[L - 1] : __int_as_float(0x7f800000);
-            uint64_t    key[SPL];
-            bool        keep[SPL];
+            const uint32_t tail = n == L ? __float_as_uint(wl_d[L - 1]) : kNone;
+            uint64_t       key[SPL];
+            bool           keep[SPL];
 #pragma unroll
             for (int s = 0; s < SPL; ++s) {
                 uint32_t j = (uint32_t)s * 32u + lane;
@@ -203,7 +207,7 @@ __global__ void __launch_bounds__(128, MINB) search_kernel(SearchArgs a) {
                 key[s]     = ~0ull;
                 if (j < cnt) {
                     float dd = nb_d[j];
-                    keep[s]  = n < L || dd < tail;
+                    keep[s]  = __float_as_uint(dd) < tail;
                     key[s]   = make_key(dd, nb_id[j]);
                 }
             }
@@ -264,7 +268,7 @@ __global__ void __launch_bounds__(128, MINB) search_kernel(SearchArgs a) {
                 }
             }
             const float    d_e      = e_pos != kNone ? wl_d[e_pos] : __int_as_float(0x7f800000);
-            const bool     take_new = kc > 0 && nb_d[0] < d_e;
+            const bool     take_new = kc > 0 && __float_as_uint(nb_d[0]) < __float_as_uint(d_e);
             const bool     has_next = take_new || e_pos != kNone;
             const uint32_t next     = take_new ? nb_id[0] : (has_next ? (wl_id[e_pos] & ~kVisitedBit) : 0u);
             const float    next_d   = take_new ? nb_d[0] : d_e;
@@ -279,7 +283,7 @@ __global__ void __launch_bounds__(128, MINB) search_kernel(SearchArgs a) {
 #pragma unroll
                 for (int s = 0; s < SPL; ++s) {
                     uint32_t j = (uint32_t)s * 32u + lane;
-                    pj[s]      = j < kc ? j + upper_bound_f(wl_d, n, nb_d[j]) : L;
+                    pj[s]      = j < kc ? j + upper_bound_f(wl_d, n, __float_as_uint(nb_d[j])) : L;
                 }
                 p0 = __shfl_sync(0xffffffffu, pj[0], 0);
                 if (p0 < L) {
@@ -292,7 +296,7 @@ __global__ void __launch_bounds__(128, MINB) search_kernel(SearchArgs a) {
                             if (i < n) {
                                 id = wl_id[i];
                                 dd = wl_d[i];
-                                np = i + lower_bound_f(nb_d, kc, dd);
+                                np = i + lower_bound_f(nb_d, kc, __float_as_uint(dd));
                             }
                             __syncwarp();
                             if (np < L) {

@@ -1,0 +1,55 @@
+"""Rows with a NaN in them sort behind every other row: a search over an index that holds
+some gives what it gives when those rows are infinitely far away instead."""
+import numpy as np
+import pytest
+
+from vann import workload
+
+pytestmark = pytest.mark.gpu
+
+N, BAD = 900, 150
+
+
+def _graphs(vann_mod, D, R, stores):
+    """Two indexes over one graph: every tenth row NaN in one, of distance +inf in the other."""
+    import torch
+
+    base = workload.mixture(N, D, 12, seed=401)
+    idx = vann_mod.Index(D, R, 48, 1.2, capacity=N)
+    idx.build(torch.from_numpy(base).cuda(), batch=0, seed=5)
+    entry = idx.info()["entry"]
+    _, deg, adj = idx.get_graph()
+    rng = np.random.default_rng(7)
+    bad = np.setdiff1d(rng.permutation(N), [entry], assume_unique=True)[:BAD]
+    out = []
+    for value in (np.nan, 3e38):
+        rows = base.copy()
+        rows[bad, 1] = value
+        i = vann_mod.Index(D, R, 48, 1.2, capacity=N, stores=stores)
+        i.set_graph(rows, deg, adj, entry)
+        out.append(i)
+    return out, bad
+
+
+def _same(vann_mod, pair, bad, nq, D, **kw):
+    import torch
+
+    q = torch.from_numpy(workload.mixture(nq, D, 12, seed=402)).cuda()
+    (ids, d, st), (ids2, d2, st2) = (i.search_stats(q, **kw) for i in pair)
+    assert torch.equal(ids, ids2) and torch.equal(st, st2)
+    far = torch.isin(ids, torch.from_numpy(bad.astype(np.int32)).cuda())
+    assert bool(torch.isnan(d[far]).all()) and bool(torch.isinf(d2[far]).all())
+    assert torch.equal(d[~far], d2[~far])
+    return far
+
+
+@pytest.mark.parametrize("D,R,L,store,rerank", [(32, 32, 100, "f32", False), (128, 64, 65, "bf16", True),
+                                                (32, 64, 1000, "f32", False), (128, 96, 40, "f32", False),
+                                                (160, 64, 300, "f32", True), (384, 20, 40, "bf16", False)])
+def test_warp_per_query_lists(vann_mod, D, R, L, store, rerank):
+    import torch
+
+    nq = 7 * torch.cuda.get_device_properties(0).multi_processor_count + 64  # too many for a CTA per query
+    pair, bad = _graphs(vann_mod, D, R, ("f32", store) if store != "f32" else ("f32",))
+    far = _same(vann_mod, pair, bad, nq, D, k=L, L=L, store=store, rerank=rerank)
+    assert L < 1000 or bool(far.any())  # long lists reach the far rows
