@@ -74,6 +74,7 @@ __global__ void __launch_bounds__(kCtaThreads, LREG <= 4 ? 4 : 3) search_cta_ker
     constexpr uint32_t    SLOTS = SPL * 32;
     constexpr uint32_t    kDone = 0xFFFFFFFFu;
     const float           kInf  = __int_as_float(0x7f800000);
+    const uint32_t        open  = strict ? __float_as_uint(kInf) : kNone;  // tail of a list with room
     const uint32_t        tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     const CtaSearchLayout lay   = CtaSearchLayout::make(a.L, SLOTS, a.rerank != 0);
     uint32_t*             bloom = reinterpret_cast<uint32_t*>(smem);
@@ -83,7 +84,8 @@ __global__ void __launch_bounds__(kCtaThreads, LREG <= 4 ? 4 : 3) search_cta_ker
     uint64_t*             skey  = reinterpret_cast<uint64_t*>(smem + lay.srt);
     uint64_t*             keys  = reinterpret_cast<uint64_t*>(smem + lay.keys);
     // [0] query, [1] entry distance, then the worklist's length, [4 + 4 p ..] what the
-    // worklist tells hop p: first unvisited entry (id, distance), tail distance, full;
+    // worklist tells hop p: first unvisited entry (id, distance), tail distance (as bits:
+    // both sides order distances by their bits, a NaN behind +inf);
     // [12 + 4 p ..] candidates in each segment of 32 slots of the hop (kDone: no hop)
     uint32_t*             ctl  = reinterpret_cast<uint32_t*>(smem + lay.ctl);
     uint32_t*             seg  = ctl + 12;
@@ -107,7 +109,7 @@ __global__ void __launch_bounds__(kCtaThreads, LREG <= 4 ? 4 : 3) search_cta_ker
             // the end) and id | visited.
             uint32_t parent = entry, hops = 0, nv = 0, p = 0;
             float    pd = __uint_as_float(ctl[1]);
-            float    e_d = kInf;  // the first unvisited entry, as the others know it
+            uint32_t e_d  = __float_as_uint(kInf);  // the first unvisited entry, as the others know it
             bool     e_in = false;
             uint32_t wd[LREG], wp[LREG];
 #pragma unroll
@@ -122,8 +124,7 @@ __global__ void __launch_bounds__(kCtaThreads, LREG <= 4 ? 4 : 3) search_cta_ker
                 wl_d[0]  = pd;
                 ctl[4]   = kNone;
                 ctl[5]   = __float_as_uint(kInf);
-                ctl[6]   = __float_as_uint(L == 1u ? pd : kInf);
-                ctl[7]   = L == 1u ? 1u : 0u;
+                ctl[6]   = L == 1u ? __float_as_uint(pd) : open;
             }
             __syncwarp();
             for (;;) {
@@ -140,15 +141,14 @@ __global__ void __launch_bounds__(kCtaThreads, LREG <= 4 ? 4 : 3) search_cta_ker
                 const float*    nb_d  = reinterpret_cast<const float*>(nb_id + SLOTS);
 
                 // the candidates that can enter
-                const bool  full = n == L;
-                const float tail = full ? wl_d[L - 1] : kInf;
-                uint32_t    kc = 0, best = kNone;
+                const uint32_t tail = n == L ? __float_as_uint(wl_d[L - 1]) : open;
+                uint32_t       kc = 0, best = kNone;
 #pragma unroll
                 for (int s = 0; s < SPL; ++s) {
                     const uint32_t j    = (uint32_t)s * 32u + lane;
                     const float    dd   = nb_d[j];
                     const uint32_t id   = nb_id[j];
-                    const bool     keep = lane < seg[4u * p + s] && ((!full && !strict) || dd < tail);
+                    const bool     keep = lane < seg[4u * p + s] && __float_as_uint(dd) < tail;
                     const uint32_t m    = __ballot_sync(0xffffffffu, keep);
                     if (keep) {
                         best = min(best, __float_as_uint(dd));
@@ -236,17 +236,16 @@ __global__ void __launch_bounds__(kCtaThreads, LREG <= 4 ? 4 : 3) search_cta_ker
                 // the same rule as theirs, so that both sides stop at the same hop (a new
                 // candidate at +inf is no parent)
                 best = __reduce_min_sync(0xffffffffu, best);
-                if ((!e_in && !(__uint_as_float(best) < e_d)) || hops >= a.max_hops) break;
+                if ((!e_in && best >= e_d) || hops >= a.max_hops) break;
                 e_in = u[1] != kNone;
-                e_d  = e_in ? wl_d[u[1]] : kInf;
+                e_d  = __float_as_uint(e_in ? wl_d[u[1]] : kInf);
                 parent = wl_id[u[0]];
                 pd     = wl_d[u[0]];
                 p ^= 1u;
                 if (lane == 0) {
                     uint32_t* o = ctl + 4 + 4u * p;
                     *reinterpret_cast<uint4*>(o) =
-                        make_uint4(e_in ? wl_id[u[1]] : kNone, __float_as_uint(e_d),
-                                   __float_as_uint(n == L ? wl_d[L - 1] : kInf), n == L ? 1u : 0u);
+                        make_uint4(e_in ? wl_id[u[1]] : kNone, e_d, n == L ? __float_as_uint(wl_d[L - 1]) : open, 0u);
                 }
 #pragma unroll
                 for (int r = 0; r < LREG; ++r)
@@ -342,22 +341,19 @@ __global__ void __launch_bounds__(kCtaThreads, LREG <= 4 ? 4 : 3) search_cta_ker
                 if (ctrl) {
                     // next parent: the best candidate that can enter, or the first unvisited
                     // entry, whichever is closer (the entry on equal distance)
-                    const uint4 st   = *reinterpret_cast<const uint4*>(ctl + 4 + 4u * p);
-                    const float tail = __uint_as_float(st.z);
-                    const bool  open = st.w == 0u && !strict;
+                    const uint4 st = *reinterpret_cast<const uint4*>(ctl + 4 + 4u * p);
                     uint32_t    bd = kNone, bi = kNone;
 #pragma unroll
                     for (int s = 0; s < SPL; ++s) {
                         const uint32_t j  = (uint32_t)s * 32u + lane;
-                        const float    d  = nb_d[j];
-                        const uint32_t id = nb_id[j], u = __float_as_uint(d);
-                        const bool     in = lane < c[s] && (open || d < tail) && (u < bd || (u == bd && id < bi));
+                        const uint32_t id = nb_id[j], u = __float_as_uint(nb_d[j]);
+                        const bool     in = lane < c[s] && u < st.z && (u < bd || (u == bd && id < bi));
                         bd                = in ? u : bd;
                         bi                = in ? id : bi;
                     }
                     const uint32_t md = __reduce_min_sync(0xffffffffu, bd);
                     const uint32_t mi = __reduce_min_sync(0xffffffffu, bd == md ? bi : kNone);
-                    parent = mi != kNone && __uint_as_float(md) < __uint_as_float(st.y) ? mi : st.x;
+                    parent = mi != kNone && md < st.y ? mi : st.x;
                     if (parent != kNone) fetch_row(parent);
                 }
                 p ^= 1u;

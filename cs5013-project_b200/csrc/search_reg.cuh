@@ -282,14 +282,15 @@ __global__ void __launch_bounds__(128, MINB) search_kernel_rw(SearchArgs a) {
             __syncwarp();
 
             // keep the candidates that can enter the list, compacted to nb_key
-            float tail = __int_as_float(0x7f800000);
+            // (by bits, as the merges order them: a NaN behind +inf)
+            uint32_t tail = 0x7f800000u;
             if (n == L) {
                 const int last = (int)L - 1;
                 uint64_t  mine = wk[0];
 #pragma unroll
                 for (int r = 1; r < LREG; ++r)
                     if (r == last / 32) mine = wk[r];
-                tail = key_dist(__shfl_sync(0xffffffffu, mine, last % 32));
+                tail = (uint32_t)(__shfl_sync(0xffffffffu, mine, last % 32) >> 32);
             }
             uint64_t ckey[NS];
             bool     keep[NS];
@@ -300,7 +301,7 @@ __global__ void __launch_bounds__(128, MINB) search_kernel_rw(SearchArgs a) {
                 ckey[s]    = kSentinel;
                 if (j < cnt) {
                     float dd = nb_d[j];
-                    keep[s]  = dd < tail;
+                    keep[s]  = __float_as_uint(dd) < tail;
                     ckey[s]  = make_key(dd, nb_id[j]);
                 }
             }

@@ -53,3 +53,42 @@ def test_warp_per_query_lists(vann_mod, D, R, L, store, rerank):
     pair, bad = _graphs(vann_mod, D, R, ("f32", store) if store != "f32" else ("f32",))
     far = _same(vann_mod, pair, bad, nq, D, k=L, L=L, store=store, rerank=rerank)
     assert L < 1000 or bool(far.any())  # long lists reach the far rows
+
+
+@pytest.mark.parametrize("D,R,L,store", [(32, 32, 100, "f32"), (128, 64, 130, "f32"), (128, 64, 48, "bf16"),
+                                         (128, 128, 20, "f32"), (160, 64, 256, "bf16")])
+def test_cta_per_query(vann_mod, D, R, L, store):
+    """Small batches: as with the far rows at +inf, and as the same queries in a large batch."""
+    import torch
+
+    pair, bad = _graphs(vann_mod, D, R, ("f32", store) if store != "f32" else ("f32",))
+    _same(vann_mod, pair, bad, 40, D, k=L, L=L, store=store)
+    nq = 7 * torch.cuda.get_device_properties(0).multi_processor_count + 64
+    q = torch.from_numpy(workload.mixture(nq, D, 12, seed=402)).cuda()
+    few, all_ = (pair[0].search_stats(q[:c].contiguous(), k=L, L=L, store=store) for c in (40, nq))
+    assert torch.equal(few[0], all_[0][:40]) and torch.equal(few[2], all_[2][:, :40])
+    assert torch.equal(few[1].view(torch.int32), all_[1][:40].view(torch.int32))
+
+
+@pytest.mark.parametrize("L", [1, 12, 64, 100])
+def test_nan_entry_and_nan_query(vann_mod, L):
+    """An entry row with a NaN stays behind every other entry; a query with one ends at once."""
+    import torch
+
+    base = workload.mixture(N, 64, 12, seed=403)
+    idx = vann_mod.Index(64, 32, 48, 1.2, capacity=N)
+    idx.build(torch.from_numpy(base).cuda(), batch=0, seed=5)
+    _, deg, adj = idx.get_graph()
+    rows = base.copy()
+    rows[3, 0] = np.nan
+    idx.set_graph(rows, deg, adj, 3)
+    nq = 7 * torch.cuda.get_device_properties(0).multi_processor_count + 64
+    q = torch.from_numpy(workload.mixture(nq, 64, 12, seed=404)).cuda()
+    q[5, 9] = float("nan")
+    few, all_ = (idx.search_stats(q[:c].contiguous(), k=L, L=L) for c in (40, nq))
+    assert torch.equal(few[0], all_[0][:40]) and torch.equal(few[2], all_[2][:, :40])
+    assert torch.equal(few[1].view(torch.int32), all_[1][:40].view(torch.int32))
+    ids, d = few[0].cpu().numpy(), few[1].cpu().numpy()
+    finite = [i for i in range(40) if i != 5]
+    assert (ids[finite, 0] != 3).all() and np.isfinite(d[finite, 0]).all()
+    assert int(few[2][0, 5]) == 1  # one hop
