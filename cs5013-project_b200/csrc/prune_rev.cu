@@ -219,27 +219,30 @@ __global__ void __launch_bounds__(128) prune_rev_kernel(PruneArgs a, uint32_t* o
         //   B_j goes to j + #{i : d(A_i) <= d(B_j)},
         //   A_i to #{j : d(B_j) < d(A_i)} + #{k : (d(A_k), k) < (d(A_i), i)}.
         // A list out of order (a graph set from outside) takes the bitonic sort.
-        bool in_order = true;
-        for (uint32_t j = lane; j + 1u < nB; j += 32) in_order &= w.cd[nA + j] <= w.cd[nA + j + 1u];
+        // Distances compare by their bits, the keys' order (non-negative; a NaN sorts last: as
+        // floats it would leave a position unwritten).
+        auto dist_bits = [&](uint32_t j) { return __float_as_uint(w.cd[j]); };
+        bool in_order  = true;
+        for (uint32_t j = lane; j + 1u < nB; j += 32) in_order &= dist_bits(nA + j) <= dist_bits(nA + j + 1u);
         if (__all_sync(0xffffffffu, in_order)) {
             for (uint32_t j = lane; j < nB; j += 32) {
-                const float d   = w.cd[nA + j];
-                uint32_t    pos = j;
-                for (uint32_t i = 0; i < nA; ++i) pos += w.cd[i] <= d ? 1u : 0u;
-                w.keys[pos] = make_key(d, nA + j);
+                const uint32_t d   = dist_bits(nA + j);
+                uint32_t       pos = j;
+                for (uint32_t i = 0; i < nA; ++i) pos += dist_bits(i) <= d ? 1u : 0u;
+                w.keys[pos] = make_key(w.cd[nA + j], nA + j);
             }
             for (uint32_t i = 0; i < nA; ++i) {
-                const float di  = w.cd[i];
-                uint32_t    pos = 0;
+                const uint32_t di  = dist_bits(i);
+                uint32_t       pos = 0;
                 for (uint32_t j0 = 0; j0 < nB; j0 += 32) {
                     const uint32_t j = j0 + lane;
-                    pos += __popc(__ballot_sync(0xffffffffu, j < nB && w.cd[nA + j] < di));
+                    pos += __popc(__ballot_sync(0xffffffffu, j < nB && dist_bits(nA + j) < di));
                 }
                 for (uint32_t k = 0; k < nA; ++k) {
-                    const float dk = w.cd[k];
+                    const uint32_t dk = dist_bits(k);
                     pos += (dk < di || (dk == di && k < i)) ? 1u : 0u;
                 }
-                if (lane == 0) w.keys[pos] = make_key(di, i);
+                if (lane == 0) w.keys[pos] = make_key(w.cd[i], i);
             }
             for (uint32_t i = nc + lane; i < p2; i += 32) w.keys[i] = ~0ull;
             __syncwarp();

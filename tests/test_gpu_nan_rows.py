@@ -92,3 +92,34 @@ def test_nan_entry_and_nan_query(vann_mod, L):
     finite = [i for i in range(40) if i != 5]
     assert (ids[finite, 0] != 3).all() and np.isfinite(d[finite, 0]).all()
     assert int(few[2][0, 5]) == 1  # one hop
+
+
+@pytest.mark.parametrize("D", [32, 160])
+@pytest.mark.parametrize("R", [16, 64])
+def test_reverse_prune(vann_mod, D, R):
+    """Inserts into a graph marked consistent (reverse re-prunes by the kernel that merges
+    into lists in order) and into the same graph unmarked (every list sorted again): the
+    same lists, with NaN rows among the old and the new, and FP32 sums that round."""
+    import torch
+
+    n, m = 1200, 260
+    rng = np.random.default_rng(9)
+    base = workload.mixture(n + m, D, 12, seed=405) * np.float32(1.0009765625)
+    bad = rng.permutation(n + m)[:120]
+    base[bad, 2] = np.nan
+    entry = int(np.setdiff1d(np.arange(n), bad)[0])
+    rows = torch.from_numpy(base).cuda()
+    built = vann_mod.Index(D, R, 70, 1.2, capacity=n)
+    built.build(rows[:n], batch=0, seed=3, entry=entry)
+    _, deg, adj = built.get_graph()
+    got = []
+    for consistent in (True, False):
+        idx = vann_mod.Index(D, R, 70, 1.2, capacity=n + m)
+        idx.set_graph(base[:n], deg, adj, entry, consistent=consistent)
+        idx.insert(rows[n:])
+        got.append(idx.get_graph())
+    (_, deg_a, adj_a), (_, deg_b, adj_b) = got
+    assert np.array_equal(deg_a, deg_b)
+    live = np.arange(R) < deg_a[:, None]
+    assert np.array_equal(np.where(live, adj_a, 0), np.where(live, adj_b, 0))
+    assert (adj_a[live] < n + m).all() and np.isin(adj_a[live], bad).any()
