@@ -576,21 +576,40 @@ __device__ __forceinline__ int column_exponent(uint32_t bound_bits) {
 }
 
 // ---------------------------------------------------------------- launches
+// Lets a kernel be launched with smem bytes of dynamic shared memory (it has no static
+// ones).  The limit belongs to the function, which threads with other indexes launch at
+// other sizes: up to 48 KB nothing is needed, and above it the limit is always set to the
+// device's largest, so that no thread lowers it between another's call and its launch.
+template <typename K>
+inline cudaError_t allow_smem(K kern, size_t smem) {
+    if (smem <= 48u * 1024u) return cudaSuccess;
+    int         dev = 0, optin = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    if (e != cudaSuccess) return e;
+    if (smem > (size_t)optin) return cudaErrorInvalidValue;
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
+}
+
 // Blocks per SM of a launch, and the shared-memory carveout set to the smallest
 // one that still holds them.  The rest of the SM's unified L1/shared memory
 // stays L1, where register spills and the rows and lists that several warps
-// touch are cached.
+// touch are cached.  The carveout is a preference: another thread's launch of the same
+// kernel may change it meanwhile, which costs blocks per SM but no launch (a request that
+// fits an SM counts as one block at least).
 template <typename K>
 inline cudaError_t fit_carveout(K kern, int threads, size_t smem, int* per_sm) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
                                          (int)cudaSharedmemCarveoutMaxShared);
     if (e != cudaSuccess) return e;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, kern, threads, smem);
-    if (e != cudaSuccess || *per_sm < 1) return e;
+    if (e != cudaSuccess) return e;
     int dev = 0, cap = 0, rsv = 0;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
     if ((e = cudaDeviceGetAttribute(&cap, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev)) != cudaSuccess) return e;
     if ((e = cudaDeviceGetAttribute(&rsv, cudaDevAttrReservedSharedMemoryPerBlock, dev)) != cudaSuccess) return e;
+    if (*per_sm < 1 && smem + (size_t)rsv <= (size_t)cap) *per_sm = 1;
+    if (*per_sm < 1) return cudaSuccess;
     const size_t need = (size_t)*per_sm * (smem + (size_t)rsv);
     const int    pct  = (int)((need * 100 + (size_t)cap - 1) / (size_t)cap);
     if (pct >= 100) return cudaSuccess;

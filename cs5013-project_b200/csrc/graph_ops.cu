@@ -570,8 +570,7 @@ cudaError_t launch_consolidate_candidates(const uint32_t* deg, const uint32_t* a
     while ((1u << hbits) < 2u * cap) ++hbits;  // load factor <= 1/2
     const int    warps = 4;
     const size_t smem  = sizeof(uint32_t) * warps * (1u << hbits);
-    cudaError_t  e = cudaFuncSetAttribute(consolidate_candidates_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)smem);
+    cudaError_t  e     = allow_smem(consolidate_candidates_kernel, smem);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
     e          = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, consolidate_candidates_kernel, warps * 32, smem);

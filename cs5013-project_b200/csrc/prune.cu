@@ -227,7 +227,7 @@ cudaError_t launch_prune(const PruneArgs& a, int num_sms, cudaStream_t st) {
         kern = prune_kernel<1>;
     else
         kern = prune_kernel<2>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(kern, smem);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
     e = fit_carveout(kern, warps * 32, smem, &per_sm);

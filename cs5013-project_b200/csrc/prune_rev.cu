@@ -364,7 +364,7 @@ cudaError_t launch_prune_rev(const PruneArgs& a, bool u8, uint32_t* out_list, ui
     const size_t smem  = sizeof(RevWarp) * warps;
     auto         kern  = a.D <= 128 ? (u8 ? prune_rev_kernel<0, true> : prune_rev_kernel<0, false>)
                                     : (u8 ? prune_rev_kernel<1, true> : prune_rev_kernel<1, false>);
-    cudaError_t  e     = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t  e     = allow_smem(kern, smem);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
     e          = fit_carveout(kern, warps * 32, smem, &per_sm);

@@ -680,7 +680,7 @@ cudaError_t launch_tc(const PruneArgs& a, uint32_t* counter, const uint32_t* in_
     const size_t floor_bytes = (size_t)(per_sm_smem / (max_ctas + 1) - reserved + 1024);
     if (smem < floor_bytes) smem = floor_bytes;
     auto kern = prune_tc_kernel<MAXC, COLS, F16>;
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    e = allow_smem(kern, smem);
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
                              (int)cudaSharedmemCarveoutMaxShared);

@@ -87,7 +87,7 @@ cudaError_t launch_rerank_dc(const float* vecs, const float* q, uint64_t nq, uin
     while (Lp < L) Lp <<= 1;
     const size_t smem = (size_t)kRerankWarps * Lp * (sizeof(uint64_t) + sizeof(uint32_t));
     auto         kern = rerank_kernel<DC>;
-    cudaError_t  e    = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t  e    = allow_smem(kern, smem);
     if (e != cudaSuccess) return e;
     uint64_t grid = (nq + kRerankWarps - 1) / kRerankWarps;
     const uint64_t cap = (uint64_t)num_sms * 8u;

@@ -414,7 +414,7 @@ template <typename S, int DC, int SPL, int LREG, bool IQ>
 static cudaError_t launch_cta_t(const SearchArgs& a, int num_sms, cudaStream_t st) {
     const size_t smem = CtaSearchLayout::make(a.L, SPL * 32, a.rerank != 0).bytes;
     auto         kern = search_cta_kernel<S, DC, SPL, LREG, IQ>;
-    cudaError_t  e    = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t  e    = allow_smem(kern, smem);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
     e          = fit_carveout(kern, kCtaThreads, smem, &per_sm);

@@ -385,7 +385,7 @@ static cudaError_t launch_t(const SearchArgs& a, int num_sms, cudaStream_t st) {
     const int  warps = 4;
     size_t     smem  = (size_t)lay.bytes * warps;
     auto       kern  = search_kernel<S, DC, SPL, MINB, IQ>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(kern, smem);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
     e = fit_carveout(kern, warps * 32, smem, &per_sm);

@@ -270,7 +270,7 @@ cudaError_t launch_staged_j(const StagedArgs& a, int num_sms, cudaStream_t st) {
         warps >>= 1;
     const size_t smem = tile_bytes + (size_t)warps * warp_bytes;
     auto         kern = staged_merge_kernel<J>;
-    e                 = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    e                 = allow_smem(kern, smem);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
     e          = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, warps * 32, smem);
