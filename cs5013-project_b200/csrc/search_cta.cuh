@@ -25,7 +25,6 @@ namespace vann {
 
 constexpr uint32_t kCtaThreads = 160;  // warp 0: worklist; warps 1-4: gathers
 constexpr uint32_t kCtaGather  = 4;
-constexpr uint32_t kCtaMaxL    = 256;
 
 struct CtaSearchLayout {
     uint32_t lp;     // L rounded up to 32
