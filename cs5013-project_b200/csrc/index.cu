@@ -22,6 +22,7 @@
 #include "../../include/vann.h"
 #include "common.cuh"
 #include "kernels.h"
+#include "search_rule.h"
 
 namespace {
 
@@ -1211,34 +1212,59 @@ vann_status vann_autotune(vann_index* h, const float* d_queries, uint64_t nq, co
         h->out_tmp.ensure((sizeof(uint32_t) + sizeof(float)) * nq * sp->k);
         uint32_t*   ids = h->out_tmp.as<uint32_t>();
         float*      dd  = reinterpret_cast<float*>(ids + nq * sp->k);
-        cudaEvent_t e0, e1;
-        VCHECK(cudaEventCreate(&e0));
-        VCHECK(cudaEventCreate(&e1));
-        const auto key = std::make_tuple(sp->store, sp->rerank ? 1u : 0u, vann_index::beam_of(*sp), sp->L);
-        int   best = 0;
-        float best_ms = 1e30f;
-        for (int v = 0; v < vann::search_variants(); ++v) {
-            h->tuned[key] = v;
+        struct Events {  // destroyed on every way out
+            cudaEvent_t e[2] = {nullptr, nullptr};
+            ~Events() {
+                for (cudaEvent_t x : e)
+                    if (x) cudaEventDestroy(x);
+            }
+        } ev;
+        for (cudaEvent_t& x : ev.e) VCHECK(cudaEventCreate(&x));
+        auto timed = [&]() {  // mean ms of three searches after one that warms up
             float ms_sum = 0.f;
             for (int rep = 0; rep < 4; ++rep) {
-                VCHECK(cudaEventRecord(e0, st));
+                VCHECK(cudaEventRecord(ev.e[0], st));
                 vann_status s2 = vann_search(h, d_queries, nq, sp, ids, dd, stream);
                 VREQUIRE(s2 == VANN_OK, s2, g_last_error);
-                VCHECK(cudaEventRecord(e1, st));
-                VCHECK(cudaEventSynchronize(e1));
+                VCHECK(cudaEventRecord(ev.e[1], st));
+                VCHECK(cudaEventSynchronize(ev.e[1]));
                 float ms = 0.f;
-                VCHECK(cudaEventElapsedTime(&ms, e0, e1));
-                if (rep > 0) ms_sum += ms;  // first run warms up
+                VCHECK(cudaEventElapsedTime(&ms, ev.e[0], ev.e[1]));
+                if (rep > 0) ms_sum += ms;
             }
-            if (h_ms_out) h_ms_out[v] = ms_sum / 3.f;
-            if (ms_sum < best_ms) {
-                best_ms = ms_sum;
+            return ms_sum / 3.f;
+        };
+        const int variants = vann::search_variants();
+        // a batch for the CTA-per-query kernel has no variants: its time, and no choice made
+        // (one taken from equal runs would hold for every later large batch)
+        const vann::SearchShape shape{nq, h->p.dim, h->p.degree, sp->L, vann_index::beam_of(*sp), (int)sp->store, false};
+        if (vann::cta_per_query(shape, h->num_sms)) {
+            const float ms = timed();
+            for (int v = 0; h_ms_out && v < variants; ++v) h_ms_out[v] = ms;
+            return;
+        }
+        const auto key = std::make_tuple(sp->store, sp->rerank ? 1u : 0u, vann_index::beam_of(*sp), sp->L);
+        struct Choice {  // the fastest, or as before if a search fails
+            std::map<std::tuple<uint32_t, uint32_t, uint32_t, uint32_t>, int>& tuned;
+            const std::tuple<uint32_t, uint32_t, uint32_t, uint32_t>&          key;
+            int                                                                 v;
+            ~Choice() {
+                if (v < 0) tuned.erase(key);
+                else tuned[key] = v;
+            }
+        } choice{h->tuned, key, h->variant_for(*sp)};
+        float best_ms = 1e30f;
+        int   best    = 0;
+        for (int v = 0; v < variants; ++v) {
+            h->tuned[key]  = v;
+            const float ms = timed();
+            if (h_ms_out) h_ms_out[v] = ms;
+            if (ms < best_ms) {
+                best_ms = ms;
                 best    = v;
             }
         }
-        h->tuned[key] = best;
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
+        choice.v = best;
     });
 }
 

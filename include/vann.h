@@ -163,7 +163,10 @@ vann_status vann_search_stats(vann_index* index, const float* d_queries, uint64_
 /* Autotuner: times every compiled launch variant of the search kernel for this
  * (store, rerank, L) on the given queries (device time, CUDA events on
  * `stream`) and makes the fastest one the index's choice for later
- * vann_search calls with the same store, rerank and L.  Synchronises. */
+ * vann_search calls with the same store, rerank and L.  Batches too small to fill
+ * the chip run a kernel of their own without variants (up to 3 to 7 queries per
+ * SM, by L): given such a batch, every h_ms_out is that kernel's time and the
+ * index's choice stays as it was.  Synchronises. */
 vann_status vann_autotune(vann_index* index, const float* d_queries, uint64_t nq,
                           const vann_search_params* sp, float* h_ms_out, void* stream);
 /* Number of compiled search variants (length of vann_autotune's h_ms_out,

@@ -93,3 +93,17 @@ def test_small_inserts_equal_the_oracle(oracle, vann_mod):
             at += c
         _, gdeg, gadj = idx.get_graph()
         assert all(np.array_equal(gadj[i, :gdeg[i]], g.adj[i, :g.deg[i]]) for i in range(n0 + 60))
+
+
+def test_autotuning_on_a_small_batch_makes_no_choice(vann_mod):
+    """A batch for the CTA-per-query kernel has one launch variant: one time for all, where
+    a fastest of seven equal runs would be the choice of every later large batch."""
+    import torch
+
+    idx, q = _index(vann_mod, 1500, 128, 32, ("f32", "u8"))
+    qd = torch.from_numpy(q).cuda()
+    for store in ("f32", "u8"):
+        ms = idx.autotune(qd[:64].contiguous(), k=10, L=48, store=store)
+        assert len(set(ms)) == 1 and ms[0] > 0
+    with pytest.raises(vann_mod.VannError):
+        idx.autotune(qd, k=10, L=5)  # k > L
