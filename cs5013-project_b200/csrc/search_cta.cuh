@@ -60,6 +60,9 @@ struct CtaRows {
 __device__ __forceinline__ void gather_barrier() {
     asm volatile("bar.sync 1, %0;" ::"n"(32 * kCtaGather) : "memory");
 }
+// all warps, from the worklist's side and the gathering side: not __syncthreads, which every
+// thread must reach at the same place
+__device__ __forceinline__ void hop_barrier() { asm volatile("bar.sync 2, %0;" ::"n"(kCtaThreads) : "memory"); }
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
 // IQ: as in search_kernel.  strict: candidates enter only when strictly closer than the
@@ -102,7 +105,7 @@ __global__ void __launch_bounds__(kCtaThreads, LREG <= 4 ? 4 : 3) search_cta_ker
         uint32_t       n = 1;  // worklist entries (warp 0)
 
         if (warp == 0) {
-            __syncthreads();  // the entry's distance
+            hop_barrier();  // the entry's distance
             // initializeWorklist: entry visited, distance computed, not in the filter.  Entry
             // e of the list is in lane e % 32, register e / 32: distance bits (kNone past
             // the end) and id | visited.
@@ -135,7 +138,7 @@ __global__ void __launch_bounds__(kCtaThreads, LREG <= 4 ? 4 : 3) search_cta_ker
                     }
                     ++nv;
                 }
-                __syncthreads();  // the hop's distances are there
+                hop_barrier();  // the hop's distances are there
                 const uint32_t* nb_id = nbuf + 2u * SLOTS * p;
                 const float*    nb_d  = reinterpret_cast<const float*>(nb_id + SLOTS);
 
@@ -277,7 +280,7 @@ __global__ void __launch_bounds__(kCtaThreads, LREG <= 4 ? 4 : 3) search_cta_ker
                     dist_group<S, DC, IQ, M>(qv, a.store, a.scale, [&](int) { return entry; }, 1, a.D, lane);
                 if (lane == 0) ctl[1] = __float_as_uint(d0);
             }
-            __syncthreads();  // the entry's distance
+            hop_barrier();  // the entry's distance
             for (;;) {
                 uint32_t* nb_id = nbuf + 2u * SLOTS * p;
                 float*    nb_d  = reinterpret_cast<float*>(nb_id + SLOTS);
@@ -336,7 +339,7 @@ __global__ void __launch_bounds__(kCtaThreads, LREG <= 4 ? 4 : 3) search_cta_ker
                     const uint32_t vi = round_row_of_lane<S, DC, M>(lane);
                     if (round_writer<S, DC, M>(lane) && (int)vi < gc) nb_d[slot_of(g0 + vi)] = y;
                 }
-                __syncthreads();  // the distances are there, and the previous merge is done
+                hop_barrier();  // the distances are there, and the previous merge is done
                 if (ctrl) {
                     // next parent: the best candidate that can enter, or the first unvisited
                     // entry, whichever is closer (the entry on equal distance)
