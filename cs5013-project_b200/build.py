@@ -25,7 +25,7 @@ SOURCES = ["search.cu", "search_f32.cu", "search_bf16.cu", "search_fp8.cu", "sea
            "prune_tc.cu", "prune_rev.cu", "staged.cu", "formats.cu", "graph_ops.cu", "index.cu", "server.cu",
            "rerank.cu"]
 HEADERS = ["common.cuh", "kernels.h", "search_impl.cuh", "search_reg.cuh", "search_cta.cuh", "search_dispatch.cuh",
-           "gram_tiles.h", "search_rule.h"]
+           "search_rule.h"]
 
 
 def _stale(obj: str, src: str) -> bool:

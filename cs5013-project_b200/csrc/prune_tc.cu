@@ -47,7 +47,6 @@
 #include <cuda_fp16.h>
 
 #include "common.cuh"
-#include "gram_tiles.h"
 #include "kernels.h"
 
 namespace vann {
@@ -459,6 +458,7 @@ __global__ void __launch_bounds__(tc_threads(MAXC), MAXC == 128 ? 8 : (MAXC == 2
         __syncthreads();
 
         // --- 4. Gram tiles on the tensor cores; squared norms of the staged rows
+        const uint32_t nb = (m + 127u) / 128u;  // row blocks of 128
         auto issue_tile = [&](uint32_t r, uint32_t c) {
             const uint32_t left = m - COLS * c;
             const uint32_t N    = ((left < COLS ? left : COLS) + 15u) & ~15u;
@@ -486,59 +486,59 @@ __global__ void __launch_bounds__(tc_threads(MAXC), MAXC == 128 ? 8 : (MAXC == 2
             __syncthreads();
         }
 
-        // --- 5. bits of the candidates that prune t
-        // "u prunes t" is alpha * d(u, t) <= d(node, t) in FP32, with d(u, t) the exact
-        // integer Y = |u|^2 + |t|^2 - 2 u.t (< 2^24, so FP32 holds it exactly).  fl(Y *
-        // alpha) does not decrease as Y grows, so the test is Y <= Ymax(t), the largest
-        // integer with fl(Ymax * alpha) <= d(node, t): 2 u.t - |u|^2 >= |t|^2 - Ymax(t).
-        // Float rows: with the Gram entry g of the f16 rows, d(u, t) is su + st - g2 g up
-        // to an error E, so u prunes t for certain where g2 g - su > st - st / alpha + E,
-        // and for certain not where it is < st - st / alpha - E (su <= st: u comes first).
-        // E: f16 rounding of both rows (2^-11 of each component) and the tensor core's
-        // FP32 accumulation, 2 (2^-10 + 2^-15) sqrt(su st) <= 0.00202 st; the FP32 sums
-        // su, st and d(u, t) themselves and this test's arithmetic, 4e-5 st; f16
-        // subnormals, 1e-9 of the longest row; FP32 subnormals, 1e-37.
-        uint32_t t = 0, last = 0;  // this thread's candidate of the row block, the warp's last one
-        int      thr  = 0;
-        float    flo = 0.f, fhi = 0.f;
-        uint32_t keep = ~0u;  // consistent lists: no B candidate is checked against another
-        const bool arrived = gram_tiles<COLS>(
-            m,
-            [&](uint32_t r) {
-                t    = 128u * r + (tid & 127u);
-                last = 128u * r + 32u * (warp & 3u) + 31u;
-                thr  = 0;
-                flo  = fhi = 0.f;
-                keep = ~0u;
-                if (t < m) {
-                    const float sdt = sd[t];
-                    if constexpr (F16) {
-                        const float mid = sdt - sdt / a.alpha;
-                        const float err = 0.0022f * sdt + slack + 1e-37f;
-                        flo             = mid - err;
-                        fhi             = mid + err;
-                    } else {
-                        int y = (int)fminf(floorf(sdt / a.alpha), 16777215.f);
-                        while (y < 16777215 && (float)(y + 1) * a.alpha <= sdt) ++y;
-                        while (y > 0 && (float)y * a.alpha > sdt) --y;
-                        thr = (int)nrm[t] - y;
+        // --- 5. bits of the candidates that prune t.  A thread whose wait gave up neither
+        // issues a tile nor waits again, and one left waiting for a tile that was not issued
+        // gives up too: two bounds at most for the node, not one per tile (21 in the largest
+        // class).  (A vote at each tile's barrier, or the walk as a function over lambdas,
+        // made a 5% consolidation of 300k rows 10.0 -> 10.1 ms.)
+        bool late = false;
+        for (uint32_t r = 0; r < nb; ++r) {
+            const uint32_t t = 128u * r + (tid & 127u);
+            // "u prunes t" is alpha * d(u, t) <= d(node, t) in FP32, with d(u, t) the exact
+            // integer Y = |u|^2 + |t|^2 - 2 u.t (< 2^24, so FP32 holds it exactly).  fl(Y *
+            // alpha) does not decrease as Y grows, so the test is Y <= Ymax(t), the largest
+            // integer with fl(Ymax * alpha) <= d(node, t): 2 u.t - |u|^2 >= |t|^2 - Ymax(t).
+            // Float rows: with the Gram entry g of the f16 rows, d(u, t) is su + st - g2 g up
+            // to an error E, so u prunes t for certain where g2 g - su > st - st / alpha + E,
+            // and for certain not where it is < st - st / alpha - E (su <= st: u comes first).
+            // E: f16 rounding of both rows (2^-11 of each component) and the tensor core's
+            // FP32 accumulation, 2 (2^-10 + 2^-15) sqrt(su st) <= 0.00202 st; the FP32 sums
+            // su, st and d(u, t) themselves and this test's arithmetic, 4e-5 st; f16
+            // subnormals, 1e-9 of the longest row; FP32 subnormals, 1e-37.
+            int      thr  = 0;
+            float    flo = 0.f, fhi = 0.f;
+            uint32_t keep = ~0u;  // consistent lists: no B candidate is checked against another
+            if (t < m) {
+                const float sdt = sd[t];
+                if constexpr (F16) {
+                    const float mid = sdt - sdt / a.alpha;
+                    const float err = 0.0022f * sdt + slack + 1e-37f;
+                    flo             = mid - err;
+                    fhi             = mid + err;
+                } else {
+                    int y = (int)fminf(floorf(sdt / a.alpha), 16777215.f);
+                    while (y < 16777215 && (float)(y + 1) * a.alpha <= sdt) ++y;
+                    while (y > 0 && (float)y * a.alpha > sdt) --y;
+                    thr = (int)nrm[t] - y;
+                }
+                if (a.consistent && (sid[t] & kB)) keep = 0u;
+            }
+            const uint32_t last  = 128u * r + 32u * (warp & 3u) + 31u;  // the warp's last candidate
+            const uint32_t ncols = min(m, 128u * (r + 1u));
+            for (uint32_t c = 0; COLS * c < ncols; ++c) {
+                if (r != 0 || c != 0) {
+                    tc_fence_before();
+                    __syncthreads();  // every thread's reads of the previous tile are done
+                    if (tid == 0 && !late) {
+                        tc_fence_after();
+                        issue_tile(r, c);
                     }
-                    if (a.consistent && (sid[t] & kB)) keep = 0u;
                 }
-            },
-            [&](uint32_t r, uint32_t c) {
-                if (tid == 0) {
-                    tc_fence_after();
-                    issue_tile(r, c);
+                if (!late) {
+                    late = !mbar_wait(bar, phase);
+                    phase ^= 1u;
                 }
-            },
-            [&]() {
-                const bool ok = mbar_wait(bar, phase);
-                phase ^= 1u;
                 tc_fence_after();
-                return ok;
-            },
-            [&](uint32_t, uint32_t c) {
 #pragma unroll 1
                 for (uint32_t c32 = 32u * (warp >> 2); c32 < COLS; c32 += 32u * kSplit) {
                     const uint32_t u0 = COLS * c + c32;
@@ -585,13 +585,12 @@ __global__ void __launch_bounds__(tc_threads(MAXC), MAXC == 128 ? 8 : (MAXC == 2
                         }
                     }
                 }
-            },
-            [&](bool late) {
-                tc_fence_before();
-                return __syncthreads_or(late) != 0;  // and every thread's reads of the tile are done
-            });
-        if (!arrived) {
-            mbar_wait(bar, phase ^ 1u);  // bounded: the products in flight write what is freed below
+            }
+        }
+        tc_fence_before();
+        if (__syncthreads_or(late)) {  // a wait for the tensor cores gave up
+            // bounded: products still in flight write the tensor memory that is freed below
+            if (tid == 0 && late) mbar_wait(bar, phase ^ 1u);
             failed = true;
             break;
         }
