@@ -29,9 +29,9 @@
 // kernel is how many nodes an SM has in flight: up to 128 candidates a CTA takes 64
 // TMEM columns and fits 8 times (tiles of 128 x 64), larger classes 128 columns, 4 at
 // most.  Nodes with more candidates than a pass holds go to the next pass (256, 512,
-// 768), larger ones to prune_kernel.  If the uint8 copy is not exact (a device flag
-// written by the conversion kernels) this kernel returns at once and prune_kernel does
-// all.
+// 768), larger ones to prune_kernel.  The host takes these passes only when it has read
+// that the uint8 copy is exact; the device flag is checked again as a safeguard, and a
+// kernel that finds it set hands every node on.
 //
 // Float rows (F16, D <= 128): the tensor cores are a filter, the decisions stay those of
 // FP32.  The rows are staged relative to the node, scaled by a power of two and rounded
@@ -745,7 +745,10 @@ cudaError_t launch_prune_tc(const PruneArgs& a, const uint32_t* in_list, const u
     return launch_tc<768, 128>(a, counters + 3, list[0], counts + 2, out_list, out_count, n, num_sms, st);
 }
 
-// The same over float rows: passes of 128, 256 and 576 candidates.
+// The same over float rows (also exact byte rows of a length the integer passes do not
+// take): passes of 128, 256 and 576 candidates.  The 256-candidate class is resident twice per
+// SM here, but 2 to 4 nodes per SM are still better off without the 128-candidate pass: an
+// insert of 300 to 450 rows into 100k x 96 takes 0.54 ms, 0.56 with it; x 128 0.62 and 0.64.
 cudaError_t launch_prune_f16(const PruneArgs& a, const uint32_t* in_list, const uint32_t* in_count,
                              uint32_t* out_list, uint32_t* out_count, uint32_t* ws, uint32_t* counters,
                              uint32_t* counts, int num_sms, cudaStream_t st) {
